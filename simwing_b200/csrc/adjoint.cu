@@ -109,6 +109,31 @@ struct RolloutImpl {
         cuda_check(cudaMemcpyAsync(to.origin, from.origin, 3 * sizeof(double), cudaMemcpyDeviceToDevice, st), "copy");
     }
 
+    // Shared memory of the reverse kernel with hand-overs `f`: the node
+    // adjoints (with ghosts unless direct) at 0, their start adjoints, the
+    // records' multiplier and parameter adjoints, the stage descriptors where
+    // they fit, the barriers.
+    uint32_t reverse_layout(const ClusterSchedule& cs, const ClusterFlow& f, size_t limit) {
+        const uint32_t m0 = cs.kinds[0].max_cta_records, m1 = cs.kinds[1].max_cta_records;
+        uint32_t off = al16((f.direct ? cs.max_patch : cs.max_local) * 16u);
+        base.smem_vb = off; off = al16(off + cs.max_patch * 16u);
+        base.smem_lam0 = off; off = al16(off + m0 * 4u);
+        base.smem_lam1 = off; off = al16(off + m1 * 4u);
+        base.smem_acc0r = off; off = al16(off + m0 * 4u);
+        base.smem_acc0c = off; off = al16(off + m0 * 4u);
+        base.smem_acc1c = off; off = al16(off + m1 * 4u);
+        base.flow.smem_barriers = off;
+        if (!f.direct) off = al16(off + f.max_barriers * 8u);
+        base.flow.smem_bytes = off;
+        if (!f.direct) off = al16(off + f.max_barriers * 4u);
+        base.flow.smem_stages = kStagesInGlobal;
+        if (total_stages(cs) <= kSharedStages && off + total_stages(cs) * 16u <= limit) {
+            base.flow.smem_stages = off;
+            off = al16(off + total_stages(cs) * 16u);
+        }
+        return smem = off;
+    }
+
     void build(StructureImpl& s, int n_steps, int every) {
         S = &s;
         if (!S->cluster_mode)
@@ -203,25 +228,25 @@ struct RolloutImpl {
         g_comp1 = ralloc<double>(owned, r1);
         g_seg = ralloc<double>(owned, 8);
         g_mass = ralloc<double>(owned, 1);
-        // reverse kernel shared memory
-        const uint32_t P = cs.max_patch;
-        const uint32_t m0 = cs.kinds[0].max_cta_records, m1 = cs.kinds[1].max_cta_records;
-        uint32_t off = 0;
-        base.smem_xb = off; off = al16(off + P * 16u);
-        base.smem_vb = off; off = al16(off + P * 16u);
-        base.smem_lam0 = off; off = al16(off + m0 * 4u);
-        base.smem_lam1 = off; off = al16(off + m1 * 4u);
-        base.smem_acc0r = off; off = al16(off + m0 * 4u);
-        base.smem_acc0c = off; off = al16(off + m0 * 4u);
-        base.smem_acc1c = off; off = al16(off + m1 * 4u);
-        base.smem_offsets = off; off = al16(off + (cs.kinds[0].stages + cs.kinds[1].stages + 2) * 4u);
-        smem = off;
+        // reverse kernel shared memory and hand-overs
         cudaDeviceProp prop{};
         cuda_check(cudaGetDeviceProperties(&prop, S->device), "cudaGetDeviceProperties");
         const size_t limit = dynamic_smem_limit(prop);
+        ClusterFlow reverse = build_flow(S->def, cs, true, cs.forward.direct);
+        if (reverse_layout(cs, reverse, limit) > limit && !reverse.direct) {
+            reverse = build_flow(S->def, cs, true, true);
+            reverse_layout(cs, reverse, limit);
+        }
+        verify_flow(S->def, cs, reverse, true);
         if (smem > limit)
             raise(SWB_UNSUPPORTED, "the reverse sweep needs " + std::to_string(smem) +
                                        " B of shared memory per CTA; build the structure with more cluster CTAs");
+        const ClusterFlowDev offsets = base.flow;
+        base.flow = upload_flow(cs, reverse, owned, S->stream);
+        base.flow.smem_stages = offsets.smem_stages;
+        base.flow.smem_barriers = offsets.smem_barriers;
+        base.flow.smem_bytes = offsets.smem_bytes;
+        base.wait_budget = S->cparams.copy_budget;
         cuda_check(adjoint_kernel_limits(static_cast<int>(limit), S->G > 8), "adjoint kernel limits");
         cuda_check(tape_kernel_limits(static_cast<int>(limit), S->G > 8), "taping kernel limits");
         cuda_check(cudaStreamSynchronize(S->stream), "rollout setup");
@@ -306,14 +331,14 @@ struct RolloutImpl {
         return cp;
     }
 
-    cudaLaunchConfig_t config(uint32_t dyn, cudaLaunchAttribute* attr) const {
+    cudaLaunchConfig_t config(uint32_t dyn, int threads, cudaLaunchAttribute* attr) const {
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = static_cast<unsigned>(S->G);
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(static_cast<unsigned>(S->G));
-        cfg.blockDim = dim3(static_cast<unsigned>(S->threads));
+        cfg.blockDim = dim3(static_cast<unsigned>(threads));
         cfg.dynamicSmemBytes = dyn;
         cfg.stream = S->stream;
         cfg.attrs = attr;
@@ -325,7 +350,7 @@ struct RolloutImpl {
         const int K = std::min(interval, steps - c * interval);
         copy_state(ck[c], sg[0]);
         cudaLaunchAttribute attr[1];
-        const cudaLaunchConfig_t cfg = config(S->cluster_smem, attr);
+        const cudaLaunchConfig_t cfg = config(S->cluster_smem, S->threads, attr);
         for (int k = 0; k < K; ++k) {
             const ClusterParams cp = step_params(k, with_tape ? &tape[k] : nullptr);
             cuda_check(with_tape ? tape_kernel_launch(cfg, cp) : plain_cluster_launch(cfg, cp), "rollout step");
@@ -460,7 +485,7 @@ struct RolloutImpl {
         ap.ground = S->cparams.ground;
         ap.ground_normal = S->cparams.ground_normal;
         cudaLaunchAttribute attr[1];
-        const cudaLaunchConfig_t cfg = config(smem, attr);
+        const cudaLaunchConfig_t cfg = config(smem, S->reverse_threads, attr);
         int cur = 0;
         cuda_check(cudaEventRecord(ev0, st), "event");
         for (int c = segments - 1; c >= 0; --c) {

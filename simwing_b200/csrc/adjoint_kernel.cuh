@@ -287,38 +287,39 @@ __device__ __forceinline__ RecordTape load_tape(int kind, const TapeStep& tp, in
     return t;
 }
 
-__device__ __forceinline__ void reverse_record(const ClusterRecord& r, int kind, uint32_t me, uint32_t x_base,
-                                               const RecordTape& tp, float* lamb, float* acc_r, float* acc_c,
-                                               uint32_t first, float inv_dt2) {
-    const uint32_t pa = node_addr(r.ab & 0xffffu, me, 0u, x_base);
-    const uint32_t pb = node_addr(r.ab >> 16, me, 0u, x_base);
-    const uint32_t slot = r.index - first;
-    if (kind == 0) {
+// The reverse of one record of kind kKind on the CTA's node adjoints
+// (sweep_load / sweep_store: cluster_kernel.cuh); `slot`: its place among
+// the CTA's records of the kind.
+template <int kKind, int kMode>
+__device__ __forceinline__ void reverse_record(const SweepArgs& a, uint4 r, uint4 w, const RecordTape& tp, float* lamb,
+                                               float* acc_r, float* acc_c, uint32_t slot) {
+    const uint32_t sa = r.x & 0xffffu, sb = r.x >> 16;
+    const float rest = __uint_as_float(r.z), comp = __uint_as_float(r.w);
+    if constexpr (kKind == 0) {
         const float4 A4 = tp.t[0], B4 = tp.t[1];
-        const float4 XA = ld_node(pa), XB = ld_node(pb);
+        const float4 XA = sweep_load<kMode>(a, sa, w.x), XB = sweep_load<kMode>(a, sb, w.y);
         adj::DistanceGrad<float> g{v3a(XA), v3a(XB), lamb[slot], 0.0f, 0.0f};
-        adj::dist_reverse(v3a(A4), v3a(B4), XA.w, XB.w, A4.w, r.rest, fabsf(r.comp), signbit(r.comp) != 0, inv_dt2,
-                          g);
-        st_node(pa, make_float4(g.a.x, g.a.y, g.a.z, XA.w));
-        st_node(pb, make_float4(g.b.x, g.b.y, g.b.z, XB.w));
+        adj::dist_reverse(v3a(A4), v3a(B4), XA.w, XB.w, A4.w, rest, fabsf(comp), signbit(comp) != 0, a.inv_dt2, g);
+        sweep_store<kMode>(a, sa, w.x, make_float4(g.a.x, g.a.y, g.a.z, XA.w));
+        sweep_store<kMode>(a, sb, w.y, make_float4(g.b.x, g.b.y, g.b.z, XB.w));
         lamb[slot] = g.lambda;
         acc_r[slot] += g.rest;
         acc_c[slot] += g.comp;
     } else {
-        const uint32_t pc = node_addr(r.cd & 0xffffu, me, 0u, x_base);
-        const uint32_t pd = node_addr(r.cd >> 16, me, 0u, x_base);
+        const uint32_t sc = r.y & 0xffffu, sd = r.y >> 16;
         const float4 A4 = tp.t[0], B4 = tp.t[1], C4 = tp.t[2], D4 = tp.t[3];
-        const float4 XA = ld_node(pa), XB = ld_node(pb), XC = ld_node(pc), XD = ld_node(pd);
+        const float4 XA = sweep_load<kMode>(a, sa, w.x), XB = sweep_load<kMode>(a, sb, w.y),
+                     XC = sweep_load<kMode>(a, sc, w.z), XD = sweep_load<kMode>(a, sd, w.w);
         const adj::V3<float> p[4] = {v3a(A4), v3a(B4), v3a(C4), v3a(D4)};
-        const float w[4] = {XA.w, XB.w, XC.w, XD.w};
+        const float im[4] = {XA.w, XB.w, XC.w, XD.w};
         adj::DihedralGrad<float> G;
         G.p[0] = v3a(XA); G.p[1] = v3a(XB); G.p[2] = v3a(XC); G.p[3] = v3a(XD);
         G.lambda = lamb[slot];
-        adj::dihedral_reverse(p, w, A4.w, r.rest, r.comp, inv_dt2, G);
-        st_node(pa, make_float4(G.p[0].x, G.p[0].y, G.p[0].z, XA.w));
-        st_node(pb, make_float4(G.p[1].x, G.p[1].y, G.p[1].z, XB.w));
-        st_node(pc, make_float4(G.p[2].x, G.p[2].y, G.p[2].z, XC.w));
-        st_node(pd, make_float4(G.p[3].x, G.p[3].y, G.p[3].z, XD.w));
+        adj::dihedral_reverse(p, im, A4.w, rest, comp, a.inv_dt2, G);
+        sweep_store<kMode>(a, sa, w.x, make_float4(G.p[0].x, G.p[0].y, G.p[0].z, XA.w));
+        sweep_store<kMode>(a, sb, w.y, make_float4(G.p[1].x, G.p[1].y, G.p[1].z, XB.w));
+        sweep_store<kMode>(a, sc, w.z, make_float4(G.p[2].x, G.p[2].y, G.p[2].z, XC.w));
+        sweep_store<kMode>(a, sd, w.w, make_float4(G.p[3].x, G.p[3].y, G.p[3].z, XD.w));
         lamb[slot] = G.lambda;
         acc_c[slot] += G.comp;
     }
@@ -335,11 +336,12 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_adjoint_kernel_t(con
     namespace cg = cooperative_groups;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ PilotAdjoint pa;
+    __shared__ int flow_dead;
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t me = cluster.block_rank();
     const ClusterInstance& I = *p.inst;
     const int tid = threadIdx.x;
-    float4* xb = reinterpret_cast<float4*>(smem + p.smem_xb);
+    float4* xb = reinterpret_cast<float4*>(smem);
     float4* vb = reinterpret_cast<float4*>(smem + p.smem_vb);
     float* lam[2] = {reinterpret_cast<float*>(smem + p.smem_lam0), reinterpret_cast<float*>(smem + p.smem_lam1)};
     float* acc0r = reinterpret_cast<float*>(smem + p.smem_acc0r);
@@ -351,13 +353,19 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_adjoint_kernel_t(con
     const uint32_t x_base = smem_addr(xb);
     const AdjointPilot* ap = p.tape.pilot;
 
-    // stage offsets of this CTA
+    Flow flow;
+    flow_setup(flow, p.flow, me, smem, x_base, 0u, &flow_dead, I.status, p.wait_budget);
     const int S0 = I.kind[0].stages, S1 = I.kind[1].stages, S = S0 + S1;
-    uint32_t* soff = reinterpret_cast<uint32_t*>(smem + p.smem_offsets);
-    for (int i = tid; i <= S0; i += blockDim.x)
-        soff[i] = __ldg(I.kind[0].offsets + static_cast<size_t>(me) * (S0 + 1) + i);
-    for (int i = tid; i <= S1; i += blockDim.x)
-        soff[S0 + 1 + i] = __ldg(I.kind[1].offsets + static_cast<size_t>(me) * (S1 + 1) + i);
+    // this CTA's stage descriptors
+    const uint4* desc = p.flow.stages + static_cast<size_t>(me) * S;
+    if (p.flow.smem_stages != ~0u) {
+        uint4* mine = reinterpret_cast<uint4*>(smem + p.flow.smem_stages);
+        for (int i = tid; i < S; i += blockDim.x) mine[i] = __ldg(desc + i);
+        desc = mine;
+    }
+    auto kind_offset = [&](int k, int s) {
+        return __ldg(I.kind[k].offsets + static_cast<size_t>(me) * (I.kind[k].stages + 1) + s);
+    };
     // adjoint state of the step's outputs
     for (uint32_t i = tid; i < n; i += blockDim.x) {
         const float4 X = __ldg(I.pos_in + base + i);
@@ -366,8 +374,8 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_adjoint_kernel_t(con
         vb[i] = p.vb_out[base + i];
     }
     __syncthreads();
-    const uint32_t first[2] = {soff[0], soff[S0 + 1]};
-    const uint32_t count[2] = {soff[S0] - soff[0], soff[S0 + 1 + S1] - soff[S0 + 1]};
+    const uint32_t first[2] = {kind_offset(0, 0), kind_offset(1, 0)};
+    const uint32_t count[2] = {kind_offset(0, S0) - first[0], kind_offset(1, S1) - first[1]};
     // multiplier and parameter adjoints start at zero
     for (int k = 0; k < 2; ++k)
         for (uint32_t i = tid; i < count[k]; i += blockDim.x) {
@@ -383,9 +391,6 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_adjoint_kernel_t(con
     }
     if (owner && tid == 0) pa.mass = 0.0f;
     __syncthreads();
-    auto stage_lo = [&](int g) { return g < S0 ? soff[g] : soff[S0 + 1 + (g - S0)]; };
-    auto stage_hi = [&](int g) { return g < S0 ? soff[g + 1] : soff[S0 + 2 + (g - S0)]; };
-
     // ---- line-iteration Jacobians of every iteration (all warps but the
     // pilot warp, one iteration each; the pilot warp too when it is the only
     // warp); read after the cluster barriers below
@@ -439,30 +444,93 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_adjoint_kernel_t(con
         }
     }
     // ---- iterations, last first --------------------------------------------------------
-    // In the narrow instantiation each thread prefetches its first record of
-    // the next stage visited and that record's tape entries before it works on
-    // the current one, so the loads from L2 and DRAM overlap the stage and its
-    // barrier.  The record arrays' pointers are held in registers.
-    const uint4* rec[2] = {I.kind[0].rec, I.kind[1].rec};
-    ClusterRecord next;
-    next.index = ~0u;
+    // In the narrow instantiation each thread fetches its first record of the
+    // next stage visited, where its nodes go and that record's tape entries
+    // before it works on the current one, so the loads from L2 and DRAM
+    // overlap the stage and its barrier; the wide one fetches the record and
+    // where its nodes go, and loads the tape entries when it reaches them.
+    const uint4* records = I.records;
+    const bool direct = p.flow.direct != 0;
+    const uint32_t kind_first[2] = {0u, I.record_first[1]};
+    const uint32_t utid = static_cast<uint32_t>(tid), lane0 = utid & ~31u;  // the warp's first thread
+    uint4 next_stage = make_uint4(0u, 0u, 0u, 0u), next_rec = next_stage, next_send = next_stage;
     RecordTape next_tape{};
-    auto prefetch = [&](int it, int g) {
+    auto fetch = [&](int it, int g) {
+        next_stage = desc[g];
         const int kind = g < S0 ? 0 : 1;
-        next = load_record(rec[kind], stage_lo(g) + tid, stage_hi(g));
-        if (next.index != ~0u) next_tape = load_tape(kind, p.tape, it, next.index);
+        if (utid < next_stage.y) {
+            const uint32_t i = next_stage.x + utid;
+            next_rec = __ldg(records + i);
+            if constexpr (kPrefetch) next_tape = load_tape(kind, p.tape, it, i - kind_first[kind]);
+        }
+        next_send = make_uint4(0u, 0u, 0u, 0u);
+        if (utid < (next_stage.w & 0xffffu)) next_send = __ldg(p.flow.send + next_stage.z + utid);
     };
-    if (kPrefetch && p.iterations > 0 && S > 0) prefetch(p.iterations - 1, S - 1);
+    const SweepArgs args{x_base, &flow, p.inv_dt, p.inv_dt2, nullptr, nullptr, nullptr, nullptr, nullptr};
+    if (p.iterations > 0 && S > 0) fetch(p.iterations - 1, S - 1);
     // The forward ran the line iteration beside its last two stages (neither
     // touches a riser attachment node); the reverse of the line iteration runs
     // beside the reverse of those two stages, on the same idle last warp of
     // the suspension CTA: it arrives at the first reverse stage's barrier,
-    // runs, then waits, and its writes are released by its arrival at the
-    // second one's barrier.
-    const int line_stage = I.susp_cta >= 0 ? I.line_stage : -1;
+    // runs, then waits at the second one's.
+    const int line_stage = I.susp_cta >= 0 && !direct ? I.line_stage : -1;
     const bool line_warp = line_stage >= 0 && owner && (tid >> 5) == static_cast<int>(blockDim.x >> 5) - 1;
+    const int armer = blockDim.x >= 64 ? static_cast<int>(blockDim.x) - 33 : 0;
     const uint32_t slots = __ldg(I.patch_begin + p.ctas);
-    for (int it = p.iterations - 1; it >= 0; --it) {
+    uint32_t sync_id = 1, phase = 0;  // phase: reverse iterations done
+    int it = p.iterations - 1;
+    auto stage = [&]<int kKind>(int g) {
+        const uint4 d = next_stage;
+        const uint4 r = next_rec;
+        const uint4 w = next_send;
+        // the record's index of its kind, and its place among the CTA's
+        const uint32_t i = d.x + utid - kind_first[kKind], at = i - first[kKind];
+        RecordTape t;
+        if constexpr (kPrefetch)
+            t = next_tape;
+        else if (utid < d.y)
+            t = load_tape(kKind, p.tape, it, i);
+        if (g > 0)
+            fetch(it, g - 1);
+        else if (it > 0)
+            fetch(it - 1, S - 1);
+        const uint32_t edges = d.w & 0xffffu, barrier = d.w >> 16;
+        float* acc_r = kKind ? acc_c[1] : acc0r;
+        if (lane0 < edges) {
+            if (direct) {
+                if (utid < d.y) reverse_record<kKind, kDirect>(args, r, w, t, lam[kKind], acc_r, acc_c[kKind], at);
+            } else {
+                if (barrier) flow_wait(flow, barrier, phase);
+                if (utid < d.y) reverse_record<kKind, kHandOver>(args, r, w, t, lam[kKind], acc_r, acc_c[kKind], at);
+            }
+        } else if (utid < d.y) {
+            reverse_record<kKind, kInside>(args, r, w, t, lam[kKind], acc_r, acc_c[kKind], at);
+        }
+        for (uint32_t j = utid + blockDim.x; j < d.y; j += blockDim.x) {
+            const uint4 rj = __ldg(records + d.x + j);
+            const uint4 wj = j < edges ? __ldg(p.flow.send + d.z + j) : make_uint4(0u, 0u, 0u, 0u);
+            const uint32_t ij = d.x + j - kind_first[kKind];
+            const RecordTape tj = load_tape(kKind, p.tape, it, ij);
+            if (direct)
+                reverse_record<kKind, kDirect>(args, rj, wj, tj, lam[kKind], acc_r, acc_c[kKind], ij - first[kKind]);
+            else
+                reverse_record<kKind, kHandOver>(args, rj, wj, tj, lam[kKind], acc_r, acc_c[kKind], ij - first[kKind]);
+        }
+        if (direct) {
+            cluster.sync();
+        } else if (g == line_stage + 1 && line_warp) {
+            stage_arrive(sync_id);
+            line_reverse(pa, *ap, p.line_jac + static_cast<size_t>(it) * line_block, xb);
+        } else {
+            stage_sync(sync_id);
+        }
+        sync_id ^= 3u;
+        if (tid == armer) {
+            if (barrier) flow_arm(flow.bar_base + barrier * 8u, flow.bytes[barrier]);
+            if (g == S - 1 && phase > 0 && flow.home) flow_arm(flow.bar_base, flow.bytes[0]);
+        }
+    };
+    for (; it >= 0; --it, ++phase) {
         // the ground plane closed the forward iteration: a node it moved
         // kept only its position along the plane (x' = x - n (n.x - off)),
         // so its adjoint loses the normal component
@@ -478,45 +546,27 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_adjoint_kernel_t(con
                 B.z -= d * nrm.z;
                 xb[i] = B;
             }
-            cluster.sync();
+            __syncthreads();
         }
         // the line-line projections followed the pilot's line iteration
         if constexpr (kLines) {
+            cluster.sync();
             if (me == 0)
                 line_contact_reverse(*I.lines, p.tape, it,
                                      [&](uint32_t ref) { return node_addr(ref, me, 0u, x_base); });
             cluster.sync();
         }
-        if (I.susp_cta >= 0 && line_stage < 0) {
+        if (owner && line_stage < 0) {
             if (pilot_warp) line_reverse(pa, *ap, p.line_jac + static_cast<size_t>(it) * line_block, xb);
-            cluster.sync();
+            __syncthreads();
         }
-        for (int g = S - 1; g >= 0; --g) {
-            const int kind = g < S0 ? 0 : 1;
-            uint32_t i = stage_lo(g) + tid;
-            if constexpr (kPrefetch) {
-                const ClusterRecord cur = next;
-                const RecordTape cur_tape = next_tape;
-                if (g > 0)
-                    prefetch(it, g - 1);
-                else if (it > 0)
-                    prefetch(it - 1, S - 1);
-                if (cur.index != ~0u)
-                    reverse_record(cur, kind, me, x_base, cur_tape, lam[kind], kind ? acc_c[1] : acc0r, acc_c[kind],
-                                   first[kind], p.inv_dt2);
-                i += blockDim.x;
-            }
-            for (; i < stage_hi(g); i += blockDim.x)
-                reverse_record(load_record(rec[kind], i, stage_hi(g)), kind, me, x_base, load_tape(kind, p.tape, it, i),
-                               lam[kind], kind ? acc_c[1] : acc0r, acc_c[kind], first[kind], p.inv_dt2);
-            if (g == line_stage + 1 && line_warp) {
-                cluster_arrive();
-                line_reverse(pa, *ap, p.line_jac + static_cast<size_t>(it) * line_block, xb);
-                cluster_wait();
-            } else {
-                cluster.sync();
-            }
-        }
+        if (p.flow.direct && (p.ground || I.susp_cta >= 0)) cluster.sync();
+        flow_send_out(flow, p.flow, xb);
+        int g = S - 1;
+        for (; g >= S0; --g) stage.template operator()<1>(g);
+        for (; g >= 0; --g) stage.template operator()<0>(g);
+        // this CTA's node adjoints are home
+        if (flow.home) flow_wait(flow, 0, phase);
     }
     // ---- predict: x = X + dt (ref + (V + (g + f w) dt - ref) damping) --------------------
     const float vscale = p.damping * p.dt;

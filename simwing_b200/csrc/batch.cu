@@ -6,9 +6,9 @@
 // cluster schedule over g ranks (g = its node count over the target patch
 // size).  The batch packs the structures' rank ranges into clusters of C
 // ranks (first fit, largest first) and runs xpbd_cluster_packed_kernel: a CTA
-// looks up its structure and rank base in a slot table, every cluster loops
-// over the largest stage count among its structures, so all its CTAs take
-// the same barriers.
+// looks up its structure and rank base in a slot table and sweeps it at its
+// own pace; all CTAs of a cluster take the same cluster barriers outside the
+// sweep (and one per stage when a structure has a direct schedule).
 //
 // Transactions.  Per structure, buffer b (its committed state) is never
 // written during a block: the first launch reads b and writes b+1, later
@@ -51,8 +51,7 @@ struct Packing {
     int idle = 0;
     int threads = 0;
     int max_stages = 0;
-    uint32_t smem_v = 0, smem_offsets = 0, smem = 0;
-    std::vector<uint32_t> lambda_offset[3];  // per structure and kind
+    uint32_t smem = 0;
     bool membranes = false;                  // a structure carries membrane elements
 };
 
@@ -71,7 +70,7 @@ std::unique_ptr<swb_structure> build_member(const swb_structure_definition& def,
         swb_solver_options opt;
         swb_default_solver_options(&opt);
         opt.device = device;
-        opt.cluster_ctas = r;  // classic stages: a packed cluster takes the same barriers on every rank
+        opt.cluster_ctas = r;
         auto m = std::make_unique<swb_structure>();
         try {
             if (def.fabric_self_contact)
@@ -145,12 +144,12 @@ void pack(Packing& P, int cluster, int threads_opt, size_t smem_limit) {
     P.idle = 0;
     P.max_stages = 0;
     for (int c = 0; c < P.clusters; ++c) {
-        int stages = 0, seam = 0, susp = 0, guard = 0;
+        int stages = 0, direct = 0, seam = 0, guard = 0;
         for (size_t i : content[c]) {
             const StructureImpl& m = P.members[i]->s;
             stages = std::max(stages, total_stages(m.csched));
             seam = std::max(seam, m.csched.seam_stages);
-            susp |= m.def.has_suspension ? 1 : 0;
+            direct |= m.csched.forward.direct ? 1 : 0;
             guard |= m.momentum_guard ? 1 : 0;
         }
         P.max_stages = std::max(P.max_stages, stages);
@@ -168,37 +167,19 @@ void pack(Packing& P, int cluster, int threads_opt, size_t smem_limit) {
         }
         for (int r = 0; r < cluster; ++r) {
             ClusterSlot& s = P.slots[static_cast<size_t>(c) * cluster + r];
-            s.stages = stages;
+            s.stages = direct ? stages : 0;
             s.seam_stages = seam;
-            s.suspension = susp;
             s.guard = guard;
         }
     }
-    // shared memory: node arrays for the largest patch, then per-structure
-    // multipliers, then stage offsets
-    uint32_t max_patch = 0, lambda_bytes = 0, offset_bytes = 0;
+    // shared memory: a CTA lays out its own structure's
     int threads = 32;
     for (size_t i = 0; i < n; ++i) {
         const StructureImpl& m = P.members[i]->s;
-        max_patch = std::max(max_patch, m.csched.max_patch);
-        lambda_bytes = std::max(lambda_bytes, align16u(m.csched.kinds[0].max_cta_records * 4u) +
-                                                  align16u(m.csched.kinds[1].max_cta_records * 4u) +
-                                                  align16u(m.csched.kinds[2].max_cta_records * 12u));
-        offset_bytes = std::max(offset_bytes, align16u((total_stages(m.csched) + 3) * 4u));
+        P.smem = std::max(P.smem, m.cluster_smem);
         P.membranes = P.membranes || !m.def.membranes.empty();
         threads = std::max(threads, m.threads);
     }
-    P.smem_v = align16u(max_patch * 16u);
-    const uint32_t lambda_base = P.smem_v + align16u(max_patch * 16u);
-    for (int k = 0; k < 3; ++k) P.lambda_offset[k].assign(n, 0);
-    for (size_t i = 0; i < n; ++i) {
-        const StructureImpl& m = P.members[i]->s;
-        P.lambda_offset[0][i] = lambda_base;
-        P.lambda_offset[1][i] = lambda_base + align16u(m.csched.kinds[0].max_cta_records * 4u);
-        P.lambda_offset[2][i] = P.lambda_offset[1][i] + align16u(m.csched.kinds[1].max_cta_records * 4u);
-    }
-    P.smem_offsets = lambda_base + lambda_bytes;
-    P.smem = P.smem_offsets + offset_bytes;
     if (P.smem > smem_limit)
         raise(SWB_UNSUPPORTED, "batch shared memory " + std::to_string(P.smem) + " B exceeds the device limit");
     if (threads_opt > 0) threads = threads_opt;
@@ -285,9 +266,6 @@ struct BatchImpl {
                     c.origin_in = m.d_origin[in]; c.origin_out = m.d_origin[out];
                     c.status = d_status + 2 * i;
                     c.recentre = m.def.has_suspension ? 1 : 0;
-                    c.kind[0].smem_lambda = P.lambda_offset[0][i];
-                    c.kind[1].smem_lambda = P.lambda_offset[1][i];
-                    c.kind[2].smem_lambda = P.lambda_offset[2][i];
                     c.membrane_residual = m.d_mres[out];
                     rec[(i * 3 + b) * 3 + role] = c;
                 }
@@ -348,9 +326,6 @@ struct BatchImpl {
                                       st.damping_reference_velocity.z);
         cp.iterations = st.constraint_iterations;
         cp.copy_budget = 4000000000LL;
-        cp.smem_x = 0;
-        cp.smem_v = P.smem_v;
-        cp.smem_offsets = P.smem_offsets;
         if (ground.enabled) {
             cp.ground = 1;
             cp.ground_normal = make_float3(static_cast<float>(ground.normal.x), static_cast<float>(ground.normal.y),

@@ -1,0 +1,139 @@
+// Hand-over of nodes between the CTAs of a cluster (ClusterFlow,
+// cluster_schedule.h): a CTA's barriers, one per stage that receives nodes
+// and one for the nodes that come home at an iteration's end, each armed
+// with the bytes it receives per iteration.  A send is one st.async: the
+// node's 16 bytes into the receiver's node array and their count on the
+// receiver's barrier, with no fence and no wait at the sender.
+//
+// A barrier's phase p is iteration p (reverse sweeps count their own): it
+// is armed again for the next iteration only after the CTA barrier that
+// closes the receiving stage, when every thread has passed its wait.  The
+// next iteration's first nodes may be counted before that (a transaction
+// count may run ahead of its arming); the phase cannot end before the
+// arming, which is its only arrival.  A node is not overwritten before its
+// reader is done: its next value exists only after the reader's result.
+#pragma once
+
+#include "cluster_params.h"
+#include "device_common.cuh"
+
+namespace swb {
+namespace dev {
+
+struct Flow {
+    uint32_t x_base;       // shared address of the node array
+    uint32_t bar_base;     // shared address of the barriers
+    uint32_t rank_base;    // the structure's first rank in the cluster
+    const uint32_t* bytes; // per barrier (shared memory); [0]: the nodes that come home
+    uint32_t out_lo, out_hi;
+    int* dead;             // shared: a wait of this CTA ran out
+    int* status;
+    long long budget;
+    bool home;             // nodes come home to this CTA from others
+};
+
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
+    uint32_t remote;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    return remote;
+}
+
+// The CTA barrier between two stages, on one of two barrier resources so
+// that a warp that only arrives at one stage's barrier can wait at the next.
+__device__ __forceinline__ void stage_sync(uint32_t id) {
+    asm volatile("barrier.cta.sync.aligned %0, %1;" ::"r"(id), "r"(blockDim.x) : "memory");
+}
+__device__ __forceinline__ void stage_arrive(uint32_t id) {
+    asm volatile("barrier.cta.arrive.aligned %0, %1;" ::"r"(id), "r"(blockDim.x) : "memory");
+}
+
+__device__ __forceinline__ void flow_arm(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+
+// This CTA's barriers (every thread; a cluster barrier must follow before
+// the first send).
+__device__ __forceinline__ void flow_setup(Flow& f, const ClusterFlowDev& F, uint32_t me, unsigned char* smem,
+                                           uint32_t x_base, uint32_t rank_base, int* dead, int* status,
+                                           long long budget) {
+    uint32_t* bytes = reinterpret_cast<uint32_t*>(smem + F.smem_bytes);
+    f.x_base = x_base;
+    f.bar_base = smem_addr(smem + F.smem_barriers);
+    f.rank_base = rank_base;
+    f.bytes = bytes;
+    f.out_lo = __ldg(F.out_begin + me);
+    f.out_hi = __ldg(F.out_begin + me + 1);
+    f.dead = dead;
+    f.status = status;
+    f.budget = budget;
+    f.home = false;
+    if (threadIdx.x == 0) *dead = 0;
+    if (F.direct) return;
+    const uint32_t lo = __ldg(F.bytes_begin + me), n = __ldg(F.bytes_begin + me + 1) - lo;
+    for (uint32_t b = threadIdx.x; b < n; b += blockDim.x) {
+        const uint32_t v = __ldg(F.bytes + lo + b);
+        bytes[b] = v;
+        const uint32_t bar = f.bar_base + b * 8u;
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        flow_arm(bar, v);
+    }
+    f.home = n > 0 && __ldg(F.bytes + lo) > 0;
+}
+
+__device__ __forceinline__ bool flow_test(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+
+__device__ __noinline__ void flow_wait_slow(const Flow& f, uint32_t bar, uint32_t parity) {
+    const long long start = clock64();
+    while (!flow_test(bar, parity)) {
+        if (*static_cast<volatile int*>(f.dead)) return;
+        if (clock64() - start > f.budget) {
+            // later waits of this CTA return at once, so the step ends
+            *static_cast<volatile int*>(f.dead) = 1;
+            atomicOr(f.status, kStatusSyncTimeout);
+            return;
+        }
+    }
+}
+
+// Waits for phase `iteration` of this CTA's barrier `index`.
+__device__ __forceinline__ void flow_wait(const Flow& f, uint32_t index, uint32_t iteration) {
+    const uint32_t bar = f.bar_base + index * 8u;
+    if (!flow_test(bar, iteration & 1u)) flow_wait_slow(f, bar, iteration & 1u);
+}
+
+// Sends a node where its word says (cluster_schedule.h, send_word).
+__device__ __forceinline__ void flow_send(const Flow& f, uint32_t word, float4 v) {
+    const uint32_t rank = ((word >> 27) & 15u) + f.rank_base;
+    const uint32_t to = map_rank(f.x_base + (word & 0x3fffu) * 16u, rank);
+    const uint32_t bar = map_rank(f.bar_base + ((word >> 14) & 0x1fffu) * 8u, rank);
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(to),
+                 "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar)
+                 : "memory");
+}
+
+// Direct schedules: the address of a foreign node.
+__device__ __forceinline__ uint32_t flow_address(const Flow& f, uint32_t word) {
+    return map_rank(f.x_base + (word & 0x3fffu) * 16u, ((word >> 27) & 15u) + f.rank_base);
+}
+
+// The nodes this CTA sends out at the start of an iteration (every thread;
+// their values are final and visible to the block).
+__device__ __forceinline__ void flow_send_out(const Flow& f, const ClusterFlowDev& F, const float4* x) {
+    for (uint32_t e = f.out_lo + threadIdx.x; e < f.out_hi; e += blockDim.x) {
+        const uint2 o = __ldg(F.out + e);
+        flow_send(f, o.y, x[o.x]);
+    }
+}
+
+}  // namespace dev
+}  // namespace swb

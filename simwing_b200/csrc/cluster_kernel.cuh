@@ -4,15 +4,26 @@
 //
 // Same substep as xpbd_step_kernel (SoftBody::integrateSubstepTrial,
 // src/softwing/soft_body.cpp:1175-1460) with a different schedule: every
-// colour of the whole mesh is one stage, each CTA executes the stage's
-// constraints it owns, nodes of other CTAs are read and written through
-// distributed shared memory, and a cluster barrier (not a device-wide one)
-// separates stages.  A launch may carry several independent clusters; the
-// cluster index selects the instance (see ClusterInstance).
+// colour of the whole mesh is one stage, and each CTA executes the stage's
+// records it owns on its own shared memory; nodes that several CTAs touch
+// are handed from one to the next (cluster_flow.cuh).  A launch may carry
+// several independent clusters; the cluster index selects the instance (see
+// ClusterInstance).
+//
+// What bounds the sweep: a stage is one dependent chain (node loads, the
+// projection, node stores, the CTA barrier), 1,200 of them per step of the
+// full wing, with at most one record per thread.  The stage loop is
+// therefore kept short: records, send words and stage descriptors are
+// fetched one stage ahead, references are local, and no cluster barrier or
+// fence stands between two stages.  With a cluster barrier after every stage
+// and foreign nodes read and written in place, the full wing (16 CTAs) took
+// 1.93 ms a step and a 9 x 9 patch (one CTA) 0.90 ms; handed over, in blocks
+// of up to 512 threads, 1.46 ms and 0.47 ms.
 #pragma once
 
 #include <cooperative_groups.h>
 
+#include "cluster_flow.cuh"
 #include "cluster_params.h"
 #include "membrane.cuh"
 #include "contact_phase.cuh"
@@ -23,40 +34,9 @@ namespace swb {
 
 namespace dev {
 
-// `ref` names a node by (instance rank << 12 | local index); `rank_base` is
-// the instance's first rank in the cluster (0 unless several structures
-// share the cluster).
-__device__ __forceinline__ float4* node_at(uint32_t ref, uint32_t me, uint32_t rank_base, float4* x,
-                                           float4* const* peers) {
-    const uint32_t r = ref >> 12;
-    return (r == me ? x : peers[r + rank_base]) + (ref & 0xfffu);
-}
-
-// One constraint record held in registers between its prefetch and its use.
-struct ClusterRecord {
-    uint32_t ab, cd;
-    float rest, comp;
-    uint32_t index;  // record index (global), or ~0u when the slot is empty
-};
-
-__device__ __forceinline__ ClusterRecord load_record(const uint4* rec, uint32_t i, uint32_t hi) {
-    ClusterRecord r;
-    r.index = ~0u;
-    if (i < hi) {
-        const uint4 q = __ldg(rec + i);
-        r.ab = q.x;
-        r.cd = q.y;
-        r.rest = __uint_as_float(q.z);
-        r.comp = __uint_as_float(q.w);
-        r.index = i;
-    }
-    return r;
-}
-__device__ __forceinline__ ClusterRecord load_record(const ClusterKindDev& K, int, uint32_t i, uint32_t hi) {
-    return load_record(K.rec, i, hi);
-}
-
-// Cluster-window address of node `ref`: the node arrays sit at the same
+// Cluster-window address of home reference `ref` (rank << 12 | index;
+// `rank_base` is the instance's first rank in the cluster, 0 unless several
+// structures share the cluster): the node arrays sit at the same
 // shared-memory offset in every CTA, so a peer's node is this CTA's address
 // mapped to the peer's rank (mapa); a local node keeps its own address,
 // which is valid in the cluster window.
@@ -176,69 +156,147 @@ __device__ bool guard_solve(const double* m, const double* rhs, double* out) {
     return true;
 }
 
-// Projects one membrane record: its three corners through the cluster
-// window like apply_record, the step-start positions (damping) from global
-// memory by slot (pbeg = the structure's patch starts).  False when the
-// element's system has no inverse (the corners are then left as they were).
-__device__ __noinline__ bool apply_membrane(const ClusterRecord& r, uint32_t me, uint32_t rank_base,
-                                            uint32_t x_base, float* lam, uint32_t first, const float4* aux,
-                                            const float4* pos_in, const uint32_t* pbeg, float inv_dt,
-                                            float inv_dt2) {
-    const uint32_t ra = r.ab & 0xffffu, rb = r.ab >> 16, rc = r.cd & 0xffffu;
-    const uint32_t pa = node_addr(ra, me, rank_base, x_base);
-    const uint32_t pb = node_addr(rb, me, rank_base, x_base);
-    const uint32_t pc = node_addr(rc, me, rank_base, x_base);
-    float4 A = ld_node(pa), B = ld_node(pb), C = ld_node(pc);
-    const MembraneConst m = load_membrane(aux, r.index);
-    float3 PA = make_float3(0.0f, 0.0f, 0.0f), PB = PA, PC = PA;
-    if (m.damping_time != 0.0f) {
-        PA = f3(__ldg(pos_in + pbeg[ra >> 12] + (ra & 0xfffu)));
-        PB = f3(__ldg(pos_in + pbeg[rb >> 12] + (rb & 0xfffu)));
-        PC = f3(__ldg(pos_in + pbeg[rc >> 12] + (rc & 0xfffu)));
-    }
-    const bool ok = project_membrane(A, B, C, PA, PB, PC, m, lam + 3 * (r.index - first), inv_dt, inv_dt2);
-    st_node(pa, A);
-    st_node(pb, B);
-    st_node(pc, C);
-    return ok;
+// Step-start position of home reference `ref` (pbeg = the structure's patch
+// starts).
+__device__ __forceinline__ float3 start_position(const float4* pos_in, const uint32_t* pbeg, uint32_t ref) {
+    return f3(__ldg(pos_in + pbeg[ref >> 12] + (ref & 0xfffu)));
 }
 
-// Projects one record.  Taping launches first store the record's inputs
-// (node positions and multiplier) at its index in this iteration's tape
-// blocks of `rtotal` entries.
-template <bool kTape = false>
-__device__ __forceinline__ void apply_record(const ClusterRecord& r, int kind, uint32_t me, uint32_t rank_base,
-                                             uint32_t x_base, float* lam, uint32_t first, float inv_dt2,
-                                             float4* tape = nullptr, uint32_t rtotal = 0) {
-    const uint32_t pa = node_addr(r.ab & 0xffffu, me, rank_base, x_base);
-    const uint32_t pb = node_addr(r.ab >> 16, me, rank_base, x_base);
-    float l = lam[r.index - first];
-    if (kind == 0) {
-        float4 A = ld_node(pa), B = ld_node(pb);
-        if constexpr (kTape) {
-            tape[r.index] = make_float4(A.x, A.y, A.z, l);
-            tape[rtotal + r.index] = B;
+// What a stage's records work on (sweep_record: `r` the record -- local
+// references, rest length, compliance --, `w` where its nodes go, `lam` its
+// multiplier, `i` its index among the structure's records of the kind).
+struct SweepArgs {
+    uint32_t x_base;  // shared address of the node array
+    const Flow* flow;
+    float inv_dt, inv_dt2;
+    // membranes
+    const float4* aux;
+    const uint2* home;
+    const float4* pos_in;
+    const uint32_t* pbeg;
+    int* status;
+};
+
+// How a record reaches its nodes: all its own CTA's; handed over (the
+// record may send nodes on); direct schedules (foreign nodes in place).
+enum SweepMode { kInside, kHandOver, kDirect };
+
+template <int kMode>
+__device__ __forceinline__ float4 sweep_load(const SweepArgs& a, uint32_t slot, uint32_t word) {
+    if constexpr (kMode == kDirect)
+        if (word) return ld_node(flow_address(*a.flow, word));
+    return ld_own(a.x_base + slot * 16u);
+}
+template <int kMode>
+__device__ __forceinline__ void sweep_store(const SweepArgs& a, uint32_t slot, uint32_t word, float4 v) {
+    if constexpr (kMode == kDirect) {
+        if (word) {
+            st_node(flow_address(*a.flow, word), v);
+            return;
         }
-        project_distance(A, B, r.rest, r.comp, l, inv_dt2);
-        st_node(pa, A);
-        st_node(pb, B);
-    } else {
-        const uint32_t pc = node_addr(r.cd & 0xffffu, me, rank_base, x_base);
-        const uint32_t pd = node_addr(r.cd >> 16, me, rank_base, x_base);
-        float4 A = ld_node(pa), B = ld_node(pb), C = ld_node(pc), D = ld_node(pd);
-        if constexpr (kTape) {
-            tape[r.index] = make_float4(A.x, A.y, A.z, l);
-            tape[rtotal + r.index] = B;
-            tape[2 * rtotal + r.index] = C;
-            tape[3 * rtotal + r.index] = D;
-        }
-        project_dihedral(A, B, C, D, r.rest, r.comp, l, inv_dt2);
-        st_node(pa, A);
-        st_node(pb, B);
-        st_node(pc, C);
-        st_node(pd, D);
     }
-    lam[r.index - first] = l;
+    // (a node sent on comes back over this store before it is read here again)
+    st_own(a.x_base + slot * 16u, v);
+    if constexpr (kMode == kHandOver)
+        if (word) flow_send(*a.flow, word, v);
+}
+
+template <int kKind, int kMode, bool kTape>
+__device__ __forceinline__ void sweep_record(const SweepArgs& a, uint4 r, uint4 w, float* lam, uint32_t i,
+                                             float4* tape, uint32_t rtotal) {
+    const uint32_t sa = r.x & 0xffffu, sb = r.x >> 16;
+    float4 A = sweep_load<kMode>(a, sa, w.x), B = sweep_load<kMode>(a, sb, w.y);
+    if constexpr (kKind == 0) {
+        float l = *lam;
+        if constexpr (kTape) {
+            tape[i] = make_float4(A.x, A.y, A.z, l);
+            tape[rtotal + i] = B;
+        }
+        const bool ok = project_distance(A, B, __uint_as_float(r.z), __uint_as_float(r.w), l, a.inv_dt2);
+        if (!ok) {
+            if constexpr (kMode != kHandOver) return;
+            A = sweep_load<kMode>(a, sa, w.x);
+            B = sweep_load<kMode>(a, sb, w.y);
+        }
+        sweep_store<kMode>(a, sa, w.x, A);
+        sweep_store<kMode>(a, sb, w.y, B);
+        if (ok) *lam = l;
+    } else if constexpr (kKind == 1) {
+        const uint32_t sc = r.y & 0xffffu, sd = r.y >> 16;
+        float4 C = sweep_load<kMode>(a, sc, w.z), D = sweep_load<kMode>(a, sd, w.w);
+        float l = *lam;
+        if constexpr (kTape) {
+            tape[i] = make_float4(A.x, A.y, A.z, l);
+            tape[rtotal + i] = B;
+            tape[2 * rtotal + i] = C;
+            tape[3 * rtotal + i] = D;
+        }
+        const bool ok = project_dihedral(A, B, C, D, __uint_as_float(r.z), __uint_as_float(r.w), l, a.inv_dt2);
+        if (!ok) {
+            if constexpr (kMode != kHandOver) return;
+            A = sweep_load<kMode>(a, sa, w.x);
+            B = sweep_load<kMode>(a, sb, w.y);
+            C = sweep_load<kMode>(a, sc, w.z);
+            D = sweep_load<kMode>(a, sd, w.w);
+        }
+        sweep_store<kMode>(a, sa, w.x, A);
+        sweep_store<kMode>(a, sb, w.y, B);
+        sweep_store<kMode>(a, sc, w.z, C);
+        sweep_store<kMode>(a, sd, w.w, D);
+        if (ok) *lam = l;
+    } else {
+        const uint32_t sc = r.y & 0xffffu;
+        float4 C = sweep_load<kMode>(a, sc, w.z);
+        const MembraneConst m = load_membrane(a.aux, i);
+        float3 PA = make_float3(0.0f, 0.0f, 0.0f), PB = PA, PC = PA;
+        if (m.damping_time != 0.0f) {
+            const uint2 h = __ldg(a.home + i);
+            PA = start_position(a.pos_in, a.pbeg, h.x & 0xffffu);
+            PB = start_position(a.pos_in, a.pbeg, h.x >> 16);
+            PC = start_position(a.pos_in, a.pbeg, h.y & 0xffffu);
+        }
+        // an element whose system has no inverse leaves its corners as they were
+        if (!project_membrane(A, B, C, PA, PB, PC, m, lam, a.inv_dt, a.inv_dt2)) atomicOr(a.status, kStatusMembrane);
+        sweep_store<kMode>(a, sa, w.x, A);
+        sweep_store<kMode>(a, sb, w.y, B);
+        sweep_store<kMode>(a, sc, w.z, C);
+    }
+}
+
+// Two distance-type records of a stage side by side on the CTA's own nodes
+// (a stage's records share no node): their two chains overlap, and the block
+// can be as narrow as the dihedral stages want it, with registers to spare
+// (full wing: 480 threads at 128 registers 1.46 ms a step, 736 threads at 80
+// registers, one record each, 1.65 ms).  `two`: there is a second one.
+template <bool kTape>
+__device__ __forceinline__ void sweep_distance_pair(const SweepArgs& a, uint4 r, uint4 s, bool two, float* lam_r,
+                                                    float* lam_s, uint32_t i, uint32_t j, float4* tape,
+                                                    uint32_t rtotal) {
+    const uint32_t ra = a.x_base + (r.x & 0xffffu) * 16u, rb = a.x_base + (r.x >> 16) * 16u;
+    const uint32_t sa = a.x_base + (s.x & 0xffffu) * 16u, sb = a.x_base + (s.x >> 16) * 16u;
+    float4 A = ld_own(ra), B = ld_own(rb), C = ld_own(sa), D = ld_own(sb);
+    float lr = *lam_r, ls = 0.0f;
+    if (two) ls = *lam_s;
+    if constexpr (kTape) {
+        tape[i] = make_float4(A.x, A.y, A.z, lr);
+        tape[rtotal + i] = B;
+        if (two) {
+            tape[j] = make_float4(C.x, C.y, C.z, ls);
+            tape[rtotal + j] = D;
+        }
+    }
+    const bool ok_r = project_distance(A, B, __uint_as_float(r.z), __uint_as_float(r.w), lr, a.inv_dt2);
+    const bool ok_s = project_distance(C, D, __uint_as_float(s.z), __uint_as_float(s.w), ls, a.inv_dt2) && two;
+    if (ok_r) {
+        st_own(ra, A);
+        st_own(rb, B);
+        *lam_r = lr;
+    }
+    if (ok_s) {
+        st_own(sa, C);
+        st_own(sb, D);
+        *lam_s = ls;
+    }
 }
 
 // Records the pilot's inputs of a line iteration (or of the finish).
@@ -285,10 +343,10 @@ __device__ __forceinline__ void ground_pass(float4* x, uint32_t n, float3 nrm, f
     }
 }
 
-// kPacked = false: one structure per cluster (cluster index = structure).
 // One load-path cable pair (soft_body.cpp:1265-1286): the levels of the
-// reverse and the forward pass over this CTA's cable and tie records, a
-// cluster barrier after each level.  Out of line: only runs with pairs.
+// reverse and the forward pass over this CTA's cable and tie records, their
+// nodes at home through the cluster window, a cluster barrier after each
+// level.  Out of line: only runs with pairs.
 __device__ __noinline__ void run_cable_pair(const ClusterInstance& I, uint32_t me, uint32_t rank_base,
                                             uint32_t x_base, float* lam0, uint32_t first0, float inv_dt2) {
     cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
@@ -297,33 +355,44 @@ __device__ __noinline__ void run_cable_pair(const ClusterInstance& I, uint32_t m
         const uint32_t hi = __ldg(off + l + 1);
         for (uint32_t i = __ldg(off + l) + threadIdx.x; i < hi; i += blockDim.x) {
             const uint32_t r = __ldg(I.pair_rec + i);
-            apply_record<false>(load_record(I.kind[0].rec, r, r + 1), 0, me, rank_base, x_base, lam0, first0,
-                                inv_dt2);
+            const uint4 q = __ldg(I.kind[0].rec + r);
+            const uint32_t ab = __ldg(&I.kind[0].home[r].x);
+            const uint32_t pa = node_addr(ab & 0xffffu, me, rank_base, x_base);
+            const uint32_t pb = node_addr(ab >> 16, me, rank_base, x_base);
+            float lam = lam0[r - first0];
+            float4 A = ld_node(pa), B = ld_node(pb);
+            if (!project_distance(A, B, __uint_as_float(q.z), __uint_as_float(q.w), lam, inv_dt2)) continue;
+            st_node(pa, A);
+            st_node(pb, B);
+            lam0[r - first0] = lam;
         }
         cluster.sync();
     }
 }
 
+// kPacked = false: one structure per cluster (cluster index = structure).
 // kPacked = true: a cluster carries several structures, each on its own
-// contiguous range of ranks, all in lockstep over the cluster's stage count;
-// the structure's buffers follow the launch role and its committed-buffer
+// contiguous range of ranks; the structure's buffers follow the launch role and its committed-buffer
 // rotation (see ClusterParams).
 // kTape = true: one structure per cluster; the step also records the inputs
 // of every projection, line iteration and the pilot finish into p.tape for
 // the reverse sweep of the adjoint.
 // kMembrane = true: the launch's structures may carry membrane elements
 // (a third record kind); without it their stage count is taken as zero.
-template <bool kPacked, bool kTape = false, bool kMembrane = false, bool kContact = false>
-__global__ void __launch_bounds__(kClusterMaxThreads) xpbd_cluster_kernel_t(const __grid_constant__ ClusterParams p) {
+// kMaxThreads: the launch bound; up to kClusterThreads threads a thread has the
+// registers the stage loop wants (see cluster_params.h), above them it spills.
+template <bool kPacked, bool kTape = false, bool kMembrane = false, bool kContact = false,
+          int kMaxThreads = kClusterThreads>
+__global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_kernel_t(const __grid_constant__ ClusterParams p) {
     static_assert(!(kContact && (kPacked || kTape)), "contact runs in single-structure forward launches only");
     namespace cg = cooperative_groups;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint64_t bar;
     __shared__ DevPayloadState pay;
     __shared__ DevPayloadDef pdef;  // suspension CTA: the payload definition, read on every line iteration
-    __shared__ float4* peers[16];
     __shared__ float3 shift_s;
     __shared__ uint32_t pbeg_s[kClusterMaxCtasDev + 1];  // the structure's patch starts
+    __shared__ int flow_dead;
     __shared__ double mom_scratch[kMaxWarps * kMomentumFields];
     __shared__ double mom_pred[kMomentumFields], mom_cur[kMomentumFields];
     __shared__ double mom_ptot[kMomentumFields], mom_tot[kMomentumFields];
@@ -355,7 +424,7 @@ __global__ void __launch_bounds__(kClusterMaxThreads) xpbd_cluster_kernel_t(cons
         slot = p.slots[blockIdx.x];
         if (slot.instance < 0) {
             // idle rank: take every cluster barrier the busy ranks take
-            const int barriers = 3 + p.iterations * (slot.stages + slot.suspension + (p.ground ? 1 : 0)) +
+            const int barriers = 4 + p.iterations * (slot.stages + (slot.stages && p.ground ? 1 : 0)) +
                                  (p.iterations > 0 ? slot.seam_stages : 0) + (slot.guard && !p.ground ? 3 : 0);
             for (int b = 0; b < barriers; ++b) cluster.sync();
             return;
@@ -367,8 +436,10 @@ __global__ void __launch_bounds__(kClusterMaxThreads) xpbd_cluster_kernel_t(cons
         kPacked ? p.instances[(static_cast<size_t>(slot.instance) * 3 + p.rotation[slot.instance]) * 3 + p.role]
                 : p.instances[blockIdx.x / p.ctas];
     const int tid = threadIdx.x;
-    float4* x = reinterpret_cast<float4*>(smem + p.smem_x);
-    float4* v = reinterpret_cast<float4*>(smem + p.smem_v);
+    float4* x = reinterpret_cast<float4*>(smem);
+    // forces and predicted velocities before the iterations, velocities
+    // after them; the multipliers lie in the same place in between
+    float4* v = reinterpret_cast<float4*>(smem + I.smem_v);
     float* lam0 = reinterpret_cast<float*>(smem + I.kind[0].smem_lambda);
     float* lam1 = reinterpret_cast<float*>(smem + I.kind[1].smem_lambda);
     float* lam2 = reinterpret_cast<float*>(smem + I.kind[2].smem_lambda);  // three per membrane record
@@ -394,18 +465,12 @@ __global__ void __launch_bounds__(kClusterMaxThreads) xpbd_cluster_kernel_t(cons
                  : 0.0f;
     const int sctas = kPacked ? slot.ctas : p.ctas;
 
-    if (tid < p.ctas) peers[tid] = cluster.map_shared_rank(x, tid);
+    Flow flow;
+    flow_setup(flow, I.flow, me, smem, x_base, rank_base, &flow_dead, I.status, p.copy_budget);
     if (tid == 0) {
         mbar_init(&bar, 1);
         mbar_expect_tx(&bar, n * 16u);
         if (n) bulk_load(x, I.pos_in + base, n * 16u, &bar);
-    }
-    // multipliers restart every substep (soft_body.cpp:1207-1218)
-    for (int k = 0; k < (kMembrane ? 3 : 2); ++k) {
-        const uint32_t* off = I.kind[k].offsets + static_cast<size_t>(me) * (I.kind[k].stages + 1);
-        const uint32_t cnt = (__ldg(off + I.kind[k].stages) - __ldg(off)) * (k == 2 ? 3u : 1u);
-        float* lam = k == 0 ? lam0 : (k == 1 ? lam1 : lam2);
-        for (uint32_t i = tid; i < cnt; i += blockDim.x) lam[i] = 0.0f;
     }
     if (tid <= sctas) pbeg_s[tid] = __ldg(I.patch_begin + tid);
     ContactCtx cctx{};
@@ -489,6 +554,15 @@ __global__ void __launch_bounds__(kClusterMaxThreads) xpbd_cluster_kernel_t(cons
         __syncthreads();
         cta_momentum_sums(x, v, n, mom_pred, mom_scratch);
     }
+    // multipliers restart every substep (soft_body.cpp:1207-1218), in the
+    // place of the forces the prediction has read
+    __syncthreads();
+    for (int k = 0; k < (kMembrane ? 3 : 2); ++k) {
+        const uint32_t* off = I.kind[k].offsets + static_cast<size_t>(me) * (I.kind[k].stages + 1);
+        const uint32_t cnt = (__ldg(off + I.kind[k].stages) - __ldg(off)) * (k == 2 ? 3u : 1u);
+        float* lam = k == 0 ? lam0 : (k == 1 ? lam1 : lam2);
+        for (uint32_t i = tid; i < cnt; i += blockDim.x) lam[i] = 0.0f;
+    }
     cluster.sync();
     if (lines) {
         line_broadphase(*lines, me, static_cast<uint32_t>(sctas), cluster, line_addr, I.status);
@@ -501,62 +575,134 @@ __global__ void __launch_bounds__(kClusterMaxThreads) xpbd_cluster_kernel_t(cons
 
     // ---- constraint iterations ------------------------------------------------
     // Stages of one iteration: distance colours, membrane colours, then
-    // dihedral colours.  Each thread prefetches its first record of the next
-    // stage before it works on the current one, so the record fetch from L2
-    // overlaps the current stage and its cluster barrier.
+    // dihedral colours.  Each thread fetches its first record of the next
+    // stage, and where its nodes go, before it works on the current one.
     const int S0 = I.kind[0].stages, S1 = I.kind[1].stages, S2 = kMembrane ? I.kind[2].stages : 0,
               S = S0 + S1 + S2;
-    const int stages_c = kPacked ? slot.stages : S;                       // cluster-wide
-    const bool susp_c = kPacked ? slot.suspension != 0 : I.susp_cta >= 0;  // cluster-wide
-    const int seam_c = kPacked ? slot.seam_stages : I.seam_stages;         // cluster-wide
-    // this CTA's stage offsets, kind by kind: [S0 + 1] distance, [S1 + 1]
-    // dihedral, [S2 + 1] membrane
-    uint32_t* soff = reinterpret_cast<uint32_t*>(smem + p.smem_offsets);
-    for (int k = 0; k < (kMembrane ? 3 : 2); ++k) {
-        const int at = k == 0 ? 0 : (k == 1 ? S0 + 1 : S0 + S1 + 2);
-        for (int i = tid; i <= I.kind[k].stages; i += blockDim.x)
-            soff[at + i] = __ldg(I.kind[k].offsets + static_cast<size_t>(me) * (I.kind[k].stages + 1) + i);
+    const int seam_c = kPacked ? slot.seam_stages : I.seam_stages;  // cluster-wide
+    // cluster barriers an iteration takes: none when every structure of the
+    // cluster hands its nodes over
+    const int stages_c = kPacked ? slot.stages : (I.flow.direct ? S : 0);
+    const uint32_t first0 = __ldg(I.kind[0].offsets + static_cast<size_t>(me) * (S0 + 1));
+    const uint32_t first1 = __ldg(I.kind[1].offsets + static_cast<size_t>(me) * (S1 + 1));
+    const uint32_t first2 = kMembrane ? __ldg(I.kind[2].offsets + static_cast<size_t>(me) * (S2 + 1)) : 0u;
+    // this CTA's stage descriptors
+    const uint4* desc = I.flow.stages + static_cast<size_t>(me) * S;
+    if (I.flow.smem_stages != ~0u) {
+        uint4* mine = reinterpret_cast<uint4*>(smem + I.flow.smem_stages);
+        for (int i = tid; i < S; i += blockDim.x) mine[i] = __ldg(desc + i);
+        desc = mine;
     }
     __syncthreads();
-    // global stage g -> kind, its stage within the kind, and its offsets
-    // (plain arithmetic: without membranes S2 is the constant 0 and these
-    // reduce to the two-kind forms)
-    auto kind_of = [&](int g) { return g < S0 ? 0 : (g < S0 + S2 ? 2 : 1); };
-    auto local_of = [&](int g) { return g < S0 ? g : (g < S0 + S2 ? g - S0 : g - S0 - S2); };
-    auto stage_at = [&](int g) {
-        return g < S0 ? g : (g < S0 + S2 ? S0 + S1 + 2 + (g - S0) : S0 + 1 + (g - S0 - S2));
+    const uint4* records = I.records;
+    const uint4* sends = I.flow.send;
+    const bool direct = I.flow.direct != 0;
+    const uint32_t kind1 = I.record_first[1], kind2 = I.record_first[2];
+    const uint32_t utid = static_cast<uint32_t>(tid), lane0 = utid & ~31u;  // the warp's first thread
+    // this stage's and the next one's descriptor, the next one's record and
+    // where its nodes go; the descriptor after that is read while they load
+    uint4 stage_now = make_uint4(0u, 0u, 0u, 0u), stage_next = stage_now, rec_next = stage_now, rec2_next = stage_now,
+          send_next = stage_now;
+    const uint32_t width = blockDim.x;
+    int ahead = 0;
+    auto read_stage = [&] {
+        const uint4 d = desc[ahead];
+        if (++ahead == S) ahead = 0;
+        return d;
     };
-    auto stage_lo = [&](int g) { return soff[stage_at(g)]; };
-    auto stage_hi = [&](int g) { return soff[stage_at(g) + 1]; };
-    const uint32_t first0 = soff[0], first1 = soff[S0 + 1], first2 = kMembrane ? soff[S0 + S1 + 2] : 0u;
-    // record arrays held in registers (the instance record lives in global memory)
-    const uint4* rec0 = I.kind[0].rec;
-    const uint4* rec1 = I.kind[1].rec;
-    const uint4* rec2 = I.kind[2].rec;
-    auto recs = [&](int k) { return k == 0 ? rec0 : (k == 1 ? rec1 : rec2); };
-    auto apply = [&](const ClusterRecord& r, int kind, float* lam, uint32_t first, float4* tape, uint32_t rtotal) {
-        if constexpr (kMembrane) {
-            if (kind == 2) {
-                if (!apply_membrane(r, me, rank_base, x_base, lam, first, I.kind[2].aux, I.pos_in, pbeg_s, p.inv_dt,
-                                    p.inv_dt2))
-                    atomicOr(I.status, kStatusMembrane);
-                return;
-            }
-        }
-        apply_record<kTape>(r, kind, me, rank_base, x_base, lam, first, p.inv_dt2, tape, rtotal);
+    auto fetch = [&](const uint4& d) {
+        if (utid < d.y) rec_next = __ldg(records + d.x + utid);
+        if (utid + width < d.y) rec2_next = __ldg(records + d.x + width + utid);
+        send_next = make_uint4(0u, 0u, 0u, 0u);
+        if (utid < (d.w & 0xffffu)) send_next = __ldg(sends + d.z + utid);
     };
-    ClusterRecord next;
-    next.index = ~0u;
-    if (p.iterations > 0 && S > 0) next = load_record(recs(kind_of(0)), stage_lo(0) + tid, stage_hi(0));
-    const uint64_t sync0 = I.kind[0].sync_mask, sync1 = I.kind[1].sync_mask;
+    SweepArgs args{x_base, &flow, p.inv_dt, p.inv_dt2, kMembrane ? I.kind[2].aux : nullptr, I.kind[2].home, I.pos_in,
+                   pbeg_s, I.status};
+    if (p.iterations > 0 && S > 0) {
+        stage_next = read_stage();
+        fetch(stage_next);
+        stage_now = stage_next;
+        stage_next = read_stage();
+    }
     // line iteration beside the last two stages: neither touches a
     // suspension endpoint node, so running it there gives the same result as
     // running it after them.  The last warp of the suspension CTA (no record
     // in either stage) arrives at the first stage's barrier, runs the line
-    // iteration, then waits; its writes are released at its arrival on the
-    // second stage's barrier, before the next iteration reads them.
-    const int line_stage = !kPacked && susp_c ? I.line_stage : -1;
+    // iteration, then waits at the second stage's; the next iteration's
+    // records read its writes after that.
+    const bool susp = I.susp_cta >= 0;
+    const int line_stage = !kPacked && susp ? I.line_stage : -1;
     const bool line_warp = line_stage >= 0 && owner && (tid >> 5) == static_cast<int>(blockDim.x >> 5) - 1;
+    // the thread that arms the barriers again: not of the last warp, which
+    // may run the line iteration, nor (with two warps or more to spare) of
+    // the first ones, which have the boundary records
+    const int armer = blockDim.x >= 64 ? static_cast<int>(blockDim.x) - 33 : 0;
+    uint32_t sync_id = 1;
+    int it = 0;
+    // One stage: its records, then the CTA barrier (a cluster barrier in a
+    // cluster with a direct schedule).
+    // `lam`: the kind's multipliers, `first` the CTA's first record of the
+    // kind (numbered over all kinds), `kind0` the kind's first record.
+    auto stage = [&]<int kKind>(int g, float* lam, uint32_t first, uint32_t kind0, float4* tape, uint32_t rtotal) {
+        const uint4 d = stage_now;
+        const uint4 r = rec_next, r2 = rec2_next;
+        const uint4 w = send_next;
+        fetch(stage_next);
+        stage_now = stage_next;
+        stage_next = read_stage();
+        const uint32_t edges = d.w & 0xffffu, barrier = d.w >> 16;
+        const uint32_t i = d.x + utid;
+        constexpr uint32_t kLam = kKind == 2 ? 3u : 1u;
+        float* lam_i = lam + kLam * (i - first);
+        const bool two = utid + width < d.y;  // a second record of the stage
+        if (lane0 < edges) {
+            if (direct) {
+                if (utid < d.y) sweep_record<kKind, kDirect, kTape>(args, r, w, lam_i, i - kind0, tape, rtotal);
+            } else {
+                if (barrier) flow_wait(flow, barrier, static_cast<uint32_t>(it));
+                if (utid < d.y) sweep_record<kKind, kHandOver, kTape>(args, r, w, lam_i, i - kind0, tape, rtotal);
+            }
+            if (two && edges <= width)
+                sweep_record<kKind, kInside, kTape>(args, r2, w, lam_i + kLam * width, i + width - kind0, tape, rtotal);
+        } else if (utid < d.y) {
+            if constexpr (kKind == 0) {
+                sweep_distance_pair<kTape>(args, r, r2, two, lam_i, lam_i + width, i, i + width, tape, rtotal);
+            } else {
+                sweep_record<kKind, kInside, kTape>(args, r, w, lam_i, i - kind0, tape, rtotal);
+                if (two)
+                    sweep_record<kKind, kInside, kTape>(args, r2, w, lam_i + kLam * width, i + width - kind0, tape,
+                                                        rtotal);
+            }
+        }
+        // stages wider than twice the block, or with more boundary records
+        // than threads
+        for (uint32_t j = utid + (edges <= width ? 2u : 1u) * width; j < d.y; j += width) {
+            const uint4 rj = __ldg(records + d.x + j);
+            const uint4 wj = j < edges ? __ldg(sends + d.z + j) : make_uint4(0u, 0u, 0u, 0u);
+            float* lj = lam + kLam * (d.x + j - first);
+            if (direct)
+                sweep_record<kKind, kDirect, kTape>(args, rj, wj, lj, d.x + j - kind0, tape, rtotal);
+            else
+                sweep_record<kKind, kHandOver, kTape>(args, rj, wj, lj, d.x + j - kind0, tape, rtotal);
+        }
+        if (stages_c) {
+            cluster.sync();
+        } else if (g == line_stage && line_warp) {
+            stage_arrive(sync_id);
+            if ((tid & 31) == 0) {
+                if constexpr (kTape) tape_pilot(p.tape.line[it], pay, *p.tape.pilot, x, nullptr);
+                line_iteration(pdef, pay, x, p.dt, I.status);
+            }
+            __syncwarp();
+        } else {
+            stage_sync(sync_id);
+        }
+        sync_id ^= 3u;
+        if (tid == armer) {
+            if (barrier) flow_arm(flow.bar_base + barrier * 8u, flow.bytes[barrier]);
+            if (g == 0 && it > 0 && flow.home) flow_arm(flow.bar_base, flow.bytes[0]);
+        }
+    };
     // load-path cable sweeps (soft_body.cpp:1288-1317): a quarter of the
     // pairs runs before the general sweeps of the first iterations, the rest
     // closes the substep (all of them without iterations)
@@ -564,64 +710,37 @@ __global__ void __launch_bounds__(kClusterMaxThreads) xpbd_cluster_kernel_t(cons
     const int closing_pairs = pairs > 0 ? pairs - pairs / 4 : 0;
     const int interleaved_pairs = pairs - closing_pairs;
     const int pair_iters = p.iterations > 1 ? p.iterations : 1;
-    for (int it = 0; it < p.iterations; ++it) {
+    for (; it < p.iterations; ++it) {
         if (pairs > 0) {
             const int n_pairs = interleaved_pairs / pair_iters + (it < interleaved_pairs % pair_iters ? 1 : 0);
+            if (n_pairs > 0) cluster.sync();  // every node is at home
             for (int q = 0; q < n_pairs; ++q) run_cable_pair(I, me, rank_base, x_base, lam0, first0, p.inv_dt2);
         }
-        for (int g = 0; g < stages_c; ++g) {
-            if (!kPacked || g < S) {
-                const int kind = kind_of(g);
-                const ClusterRecord cur = next;
-                // prefetch the next stage (wrapping to the next iteration)
-                const int gn = g + 1 < S ? g + 1 : 0;
-                next = load_record(recs(kind_of(gn)), stage_lo(gn) + tid, stage_hi(gn));
-                const uint32_t first = kind == 0 ? first0 : (kind == 1 ? first1 : first2);
-                float* lam = kind == 0 ? lam0 : (kind == 1 ? lam1 : lam2);
-                float4* tape = nullptr;
-                uint32_t rtotal = 0;
-                if constexpr (kTape) {
-                    rtotal = kind ? p.tape.r1 : p.tape.r0;
-                    tape = (kind ? p.tape.dih : p.tape.dist) + static_cast<size_t>(it) * (kind ? 4 : 2) * rtotal;
-                }
-                if (cur.index != ~0u) apply(cur, kind, lam, first, tape, rtotal);
-                for (uint32_t i = stage_lo(g) + tid + blockDim.x; i < stage_hi(g); i += blockDim.x)
-                    apply(load_record(recs(kind), i, stage_hi(g)), kind, lam, first, tape, rtotal);
-            }
-            if (g == line_stage) {
-                if (line_warp) {
-                    cluster_arrive();
-                    if ((tid & 31) == 0) {
-                        if constexpr (kTape) tape_pilot(p.tape.line[it], pay, *p.tape.pilot, x, nullptr);
-                        line_iteration(pdef, pay, x, p.dt, I.status);
-                    }
-                    __syncwarp();
-                    cluster_wait();
-                } else {
-                    cluster.sync();
-                }
-            } else if constexpr (kPacked) {
-                cluster.sync();
-            } else {
-                // split stages: a CTA barrier between two stages of records
-                // that touch only the CTA's own patch, else a cluster barrier;
-                // membrane stages are classic
-                const int kind = kind_of(g);
-                const int gl = local_of(g);
-                const uint64_t mask = kind == 0 ? sync0 : sync1;
-                if (kind == 2 || gl >= 64 || ((mask >> gl) & 1ull))
-                    cluster.sync();
-                else
-                    __syncthreads();
-            }
+        flow_send_out(flow, I.flow, x);
+        float4 *tape0 = nullptr, *tape1 = nullptr;
+        uint32_t r0 = 0, r1 = 0;
+        if constexpr (kTape) {
+            r0 = p.tape.r0;
+            r1 = p.tape.r1;
+            tape0 = p.tape.dist + static_cast<size_t>(it) * 2 * r0;
+            tape1 = p.tape.dih + static_cast<size_t>(it) * 4 * r1;
         }
-        if (susp_c && line_stage < 0) {
-            if (owner && tid == 0) {
+        int g = 0;
+        for (; g < S0; ++g) stage.template operator()<0>(g, lam0, first0, 0u, tape0, r0);
+        if constexpr (kMembrane)
+            for (; g < S0 + S2; ++g) stage.template operator()<2>(g, lam2, kind2 + first2, kind2, nullptr, 0u);
+        for (; g < S; ++g) stage.template operator()<1>(g, lam1, kind1 + first1, kind1, tape1, r1);
+        for (; g < stages_c; ++g) cluster.sync();  // packed: the cluster's longer iterations
+        if (susp && line_stage < 0 && owner) {
+            __syncthreads();
+            if (tid == 0) {
                 if constexpr (kTape) tape_pilot(p.tape.line[it], pay, *p.tape.pilot, x, nullptr);
                 line_iteration(pdef, pay, x, p.dt, I.status);
             }
-            cluster.sync();
+            __syncthreads();
         }
+        // this CTA's nodes are home
+        if (flow.home) flow_wait(flow, 0, static_cast<uint32_t>(it));
         if constexpr (kContact) contact_iteration(cctx, cluster);
         if (lines) {
             float4* line_tape = nullptr;
@@ -629,6 +748,7 @@ __global__ void __launch_bounds__(kClusterMaxThreads) xpbd_cluster_kernel_t(cons
                 if (lines->count[0] <= p.tape.line_cap)
                     line_tape = p.tape.line_in + static_cast<size_t>(it) * p.tape.line_cap * 4;
             }
+            cluster.sync();
             if (me == 0) line_project(*lines, line_addr, line_tape);
             cluster.sync();
         }
@@ -636,9 +756,13 @@ __global__ void __launch_bounds__(kClusterMaxThreads) xpbd_cluster_kernel_t(cons
             uint8_t* gt = nullptr;
             if constexpr (kTape) gt = p.tape.ground + static_cast<size_t>(it) * pbeg_s[sctas] + base;
             ground_pass(x, n, p.ground_normal, ground_off, p.ground_friction, I.pos_in + base, gt);
-            cluster.sync();
+            if (stages_c)
+                cluster.sync();
+            else
+                __syncthreads();
         }
     }
+    cluster.sync();  // every node of the cluster is home
     // closing cable pairs
     for (int q = 0; q < (p.iterations > 0 ? closing_pairs : pairs); ++q)
         run_cable_pair(I, me, rank_base, x_base, lam0, first0, p.inv_dt2);
@@ -650,17 +774,17 @@ __global__ void __launch_bounds__(kClusterMaxThreads) xpbd_cluster_kernel_t(cons
             const uint32_t hi = s < I.seam_stages ? __ldg(off + s + 1) : 0u;
             for (uint32_t i = lo + tid; i < hi; i += blockDim.x) {
                 const uint32_t r = __ldg(I.seam_ab + i);
-                float4* pa = node_at(r & 0xffffu, me, rank_base, x, peers);
-                float4* pb = node_at(r >> 16, me, rank_base, x, peers);
-                float4 A = *pa, B = *pb;
+                const uint32_t pa = node_addr(r & 0xffffu, me, rank_base, x_base);
+                const uint32_t pb = node_addr(r >> 16, me, rank_base, x_base);
+                float4 A = ld_node(pa), B = ld_node(pb);
                 if constexpr (kTape) {
                     p.tape.seam[i] = A;
                     p.tape.seam[p.tape.rs + i] = B;
                 }
                 float l = 0.0f;  // rigid stitch: alpha = 0
-                project_distance(A, B, 0.0f, 0.0f, l, p.inv_dt2);
-                *pa = A;
-                *pb = B;
+                if (!project_distance(A, B, 0.0f, 0.0f, l, p.inv_dt2)) continue;
+                st_node(pa, A);
+                st_node(pb, B);
             }
             cluster.sync();
         }
@@ -669,9 +793,9 @@ __global__ void __launch_bounds__(kClusterMaxThreads) xpbd_cluster_kernel_t(cons
     if constexpr (kContact) contact_certify(cctx, cluster, I.contact_diag);
     // ---- membrane residuals after the iterations (soft_body.cpp:2366-2404) ---
     if (kMembrane && S2 > 0) {
-        const uint32_t lo = soff[S0 + S1 + 2], hi = soff[S0 + S1 + 2 + S2];
-        for (uint32_t i = lo + tid; i < hi; i += blockDim.x) {
-            const uint4 q = __ldg(rec2 + i);
+        const uint32_t hi = __ldg(I.kind[2].offsets + static_cast<size_t>(me) * (S2 + 1) + S2);
+        for (uint32_t i = first2 + tid; i < hi; i += blockDim.x) {
+            const uint2 q = __ldg(I.kind[2].home + i);
             const uint32_t ra = q.x & 0xffffu, rb = q.x >> 16, rc = q.y & 0xffffu;
             const float4 A = ld_node(node_addr(ra, me, rank_base, x_base));
             const float4 B = ld_node(node_addr(rb, me, rank_base, x_base));
@@ -679,13 +803,14 @@ __global__ void __launch_bounds__(kClusterMaxThreads) xpbd_cluster_kernel_t(cons
             const MembraneConst m = load_membrane(I.kind[2].aux, i);
             float3 PA = make_float3(0.0f, 0.0f, 0.0f), PB = PA, PC = PA;
             if (m.damping_time != 0.0f) {
-                PA = f3(__ldg(I.pos_in + pbeg_s[ra >> 12] + (ra & 0xfffu)));
-                PB = f3(__ldg(I.pos_in + pbeg_s[rb >> 12] + (rb & 0xfffu)));
-                PC = f3(__ldg(I.pos_in + pbeg_s[rc >> 12] + (rc & 0xfffu)));
+                PA = start_position(I.pos_in, pbeg_s, ra);
+                PB = start_position(I.pos_in, pbeg_s, rb);
+                PC = start_position(I.pos_in, pbeg_s, rc);
             }
             I.membrane_residual[i] = membrane_residual(f3(A), f3(B), f3(C), PA, PB, PC, m, lam2 + 3 * (i - first2),
                                                        p.inv_dt, p.inv_dt2);
         }
+        __syncthreads();  // the velocities take the multipliers' place
     }
     // ---- finalize (soft_body.cpp:1568-1585) --------------------------------
     for (uint32_t i = tid; i < n; i += blockDim.x) {
@@ -809,17 +934,25 @@ __global__ void __launch_bounds__(kClusterMaxThreads) xpbd_cluster_kernel_t(cons
 }
 
 // One structure per cluster (the plain step) and several structures per
-// cluster (the batched step).
+// cluster (the batched step), each also with membrane elements; one structure
+// with fabric self-contact; one structure recording the adjoint's tape.  The
+// _wide forms take blocks of more than kClusterThreads threads.
 inline constexpr auto xpbd_cluster_kernel = &xpbd_cluster_kernel_t<false>;
 inline constexpr auto xpbd_cluster_packed_kernel = &xpbd_cluster_kernel_t<true>;
-// The same with membrane elements.
 inline constexpr auto xpbd_cluster_membrane_kernel = &xpbd_cluster_kernel_t<false, false, true>;
 inline constexpr auto xpbd_cluster_packed_membrane_kernel = &xpbd_cluster_kernel_t<true, false, true>;
-// One structure per cluster with fabric self-contact.
-inline constexpr auto xpbd_cluster_contact_kernel = &xpbd_cluster_kernel_t<false, false, false, true>;
-inline constexpr auto xpbd_cluster_contact_membrane_kernel = &xpbd_cluster_kernel_t<false, false, true, true>;
-// One structure per cluster, recording the adjoint's tape.
 inline constexpr auto xpbd_cluster_tape_kernel = &xpbd_cluster_kernel_t<false, true>;
+inline constexpr auto xpbd_cluster_kernel_wide = &xpbd_cluster_kernel_t<false, false, false, false, kClusterMaxThreads>;
+inline constexpr auto xpbd_cluster_packed_kernel_wide =
+    &xpbd_cluster_kernel_t<true, false, false, false, kClusterMaxThreads>;
+inline constexpr auto xpbd_cluster_membrane_kernel_wide =
+    &xpbd_cluster_kernel_t<false, false, true, false, kClusterMaxThreads>;
+inline constexpr auto xpbd_cluster_packed_membrane_kernel_wide =
+    &xpbd_cluster_kernel_t<true, false, true, false, kClusterMaxThreads>;
+inline constexpr auto xpbd_cluster_tape_kernel_wide = &xpbd_cluster_kernel_t<false, true, false, false, kClusterMaxThreads>;
+inline constexpr auto xpbd_cluster_contact_kernel = &xpbd_cluster_kernel_t<false, false, false, true, kClusterMaxThreads>;
+inline constexpr auto xpbd_cluster_contact_membrane_kernel =
+    &xpbd_cluster_kernel_t<false, false, true, true, kClusterMaxThreads>;
 
 }  // namespace dev
 }  // namespace swb

@@ -10,18 +10,17 @@
 namespace swb {
 
 namespace dev {
-constexpr int kClusterMaxThreads = 768;  // threads per CTA of the cluster step kernels
+constexpr int kClusterMaxThreads = 768;  // threads per CTA of the cluster step kernels at most
+constexpr int kClusterThreads = 512;     // ... as chosen: 128 registers a thread
 constexpr int kClusterMaxCtasDev = 16;   // CTAs per cluster at most
 }
 
 struct ClusterKindDev {
     const uint32_t* offsets;   // [ctas * (stages + 1)]
-    const uint4* rec;          // per record: ab, cd (dihedral), rest bits, compliance bits (sign = cable)
+    const uint4* rec;          // per record: local references ab, cd (dihedral), rest bits, compliance bits (sign = cable)
+    const uint2* home;         // per record: home references ab, cd (cable pairs, membranes)
     int stages;
     uint32_t smem_lambda;      // byte offset of this kind's multipliers
-    uint64_t sync_mask;        // bit g: a cluster barrier follows stage g (stages >= 64: always)
-    int interior_stages;       // stages before this one touch only the CTA's own nodes
-    int pad;
     const float4* aux;         // membranes: kMembraneAux float4 of element constants per record
 };
 
@@ -171,6 +170,18 @@ struct LineContactDev {
     uint32_t* count;                   // [2] candidate pairs of the step, their level count
 };
 
+// The hand-overs of a sweep (ClusterFlow, cluster_schedule.h).
+struct ClusterFlowDev {
+    const uint4* stages;           // [ctas * stages] stage descriptors
+    const uint4* send;             // per boundary record: where its nodes go
+    const uint32_t* bytes_begin;   // [ctas + 1]
+    const uint32_t* bytes;         // per barrier
+    const uint32_t* out_begin;     // [ctas + 1]
+    const uint2* out;              // (slot, word) of the nodes sent out at an iteration's start
+    uint32_t smem_stages, smem_barriers, smem_bytes;  // byte offsets (smem_stages ~0u: not in shared memory)
+    int direct;                    // foreign nodes in place, a cluster barrier after every stage
+};
+
 // Per-instance tables and state (one cluster each).
 struct ClusterInstance {
     const float4* pos_in;
@@ -184,6 +195,10 @@ struct ClusterInstance {
     const uint4* tri;
     const uint32_t* patch_begin;   // [ctas + 1]
     ClusterKindDev kind[3];        // distance, dihedral, membrane (swept distance, membrane, dihedral)
+    const uint4* records;          // the records of all kinds, kind[k].rec = records + record_first[k]
+    uint32_t record_first[3];
+    ClusterFlowDev flow;
+    uint32_t smem_v;               // byte offset of the force / velocity array (shares the multipliers' place)
     float* membrane_residual;      // per membrane record: normalized residual of the last substep
     const uint32_t* seam_offsets;
     const uint32_t* seam_ab;
@@ -275,9 +290,9 @@ struct TapeStep {
 struct ClusterSlot {
     int instance;      // index into the launch's structures; -1 = idle CTA
     int rank_base;     // first cluster rank of that structure
-    int stages;        // colour stages per iteration: max over the cluster
+    int stages;        // cluster barriers an iteration takes: the largest stage count when a structure
+                       // of the cluster has a direct schedule, else 0
     int seam_stages;   // seam stages: max over the cluster
-    int suspension;    // 1 when a structure of the cluster has a pilot
     int guard;         // 1 when a structure of the cluster runs the momentum guard
     int ctas;          // ranks of this CTA's structure (0 when idle)
     int pad;
@@ -296,8 +311,6 @@ struct ClusterParams {
     int iterations;
     int cable_pairs;               // load-path cable sweep pairs per substep (single-structure launches)
     long long copy_budget;
-    uint32_t smem_x, smem_v;       // byte offsets of node and force/velocity arrays
-    uint32_t smem_offsets;         // byte offset of the CTA's stage offsets
     TapeStep tape;                 // taping launches: where this step's tape goes
     // contact launches: clusters after the first that join only the contact
     // detection phases (broadphase and swept queries), synchronised with the
@@ -337,7 +350,9 @@ struct AdjointParams {
     float dt, inv_dt, inv_dt2, damping;
     float3 gravity;
     int iterations;
-    uint32_t smem_xb, smem_vb, smem_lam0, smem_lam1, smem_acc0r, smem_acc0c, smem_acc1c, smem_offsets;
+    uint32_t smem_vb, smem_lam0, smem_lam1, smem_acc0r, smem_acc0c, smem_acc1c;
+    ClusterFlowDev flow;           // the reverse sweep's hand-overs
+    long long wait_budget;         // cycles a wait for nodes may take
     int ground;                    // the frictionless ground plane of the forward step (ClusterParams)
     float3 ground_normal;
 };

@@ -325,8 +325,299 @@ static bool stage_touches(const OwnedDefinition& d, const ClusterSchedule& S, co
     return false;
 }
 
+// Global stage of stage `s` of kind k.
+static int global_stage_of(const ClusterSchedule& S, int k, int s) {
+    return k == 0 ? s : (k == 2 ? S.kinds[0].stages + s : S.kinds[0].stages + S.kinds[2].stages + s);
+}
+
+// Homes, patches and slots.  A node's home is the CTA of its first touch in
+// an iteration (its bisection part when nothing touches it, when that
+// patch is full, and in direct schedules); ghosts are the foreign nodes a
+// CTA's records touch, in node order.  `patch_limit`: nodes a patch may hold.
+static void place_nodes(ClusterSchedule& S, const std::vector<int>& part,
+                        const std::array<std::vector<std::array<uint32_t, 4>>, 3>& nodes,
+                        const std::array<std::vector<int>, 3>& counts, const std::array<std::vector<int>, 3>& cta,
+                        const std::array<std::vector<int>, 3>& colour, const std::vector<uint8_t>& attached,
+                        uint32_t patch_limit, bool direct) {
+    const uint32_t N = S.node_count;
+    const int C = S.ctas;
+    std::vector<int> home = part, first(N, -1), first_stage(N, std::numeric_limits<int>::max());
+    std::vector<uint16_t> touched(N, 0);  // CTAs that touch the node
+    for (int k = 0; k < 3; ++k)
+        for (size_t i = 0; i < counts[k].size(); ++i) {
+            const int g = global_stage_of(S, k, colour[k][i]);
+            for (int q = 0; q < counts[k][i]; ++q) {
+                const uint32_t n = nodes[k][i][q];
+                touched[n] |= static_cast<uint16_t>(1u << cta[k][i]);
+                if (g < first_stage[n]) {
+                    first_stage[n] = g;
+                    first[n] = cta[k][i];
+                }
+            }
+        }
+    std::vector<uint32_t> size(C, 0);
+    for (uint32_t n = 0; n < N; ++n) ++size[part[n]];
+    if (!direct)
+        for (uint32_t n = 0; n < N; ++n)
+            if (first[n] >= 0 && first[n] != part[n] && !attached[n] && size[first[n]] < patch_limit) {
+                --size[part[n]];
+                ++size[first[n]];
+                home[n] = first[n];
+            }
+    S.patch_begin.assign(C + 1, 0);
+    S.max_patch = 0;
+    for (int c = 0; c < C; ++c) {
+        S.max_patch = std::max(S.max_patch, size[c]);
+        S.patch_begin[c + 1] = S.patch_begin[c] + size[c];
+    }
+    S.node_of_slot.assign(N, 0);
+    S.slot_of_node.assign(N, 0);
+    std::vector<uint32_t> cur(S.patch_begin.begin(), S.patch_begin.end() - 1);
+    for (uint32_t n = 0; n < N; ++n) {
+        const uint32_t s = cur[home[n]]++;
+        S.node_of_slot[s] = n;
+        S.slot_of_node[n] = s;
+    }
+    S.ghost_begin.assign(C + 1, 0);
+    S.ghost_node.clear();
+    S.max_local = S.max_patch;
+    for (int c = 0; c < C; ++c) {
+        if (!direct)
+            for (uint32_t n = 0; n < N; ++n)
+                if (home[n] != c && (touched[n] >> c & 1)) S.ghost_node.push_back(n);
+        S.ghost_begin[c + 1] = static_cast<uint32_t>(S.ghost_node.size());
+        S.max_local = std::max(S.max_local, size[c] + S.ghost_begin[c + 1] - S.ghost_begin[c]);
+    }
+}
+
+// Home CTA of a node.
+static int home_of(const ClusterSchedule& S, uint32_t node) {
+    return static_cast<int>(std::upper_bound(S.patch_begin.begin(), S.patch_begin.end(), S.slot_of_node[node]) -
+                            S.patch_begin.begin() - 1);
+}
+
+// Slot of a node in CTA c's array (its own patch, then its ghosts).
+static uint32_t local_slot(const ClusterSchedule& S, int c, uint32_t node) {
+    const uint32_t s = S.slot_of_node[node];
+    if (s >= S.patch_begin[c] && s < S.patch_begin[c + 1]) return s - S.patch_begin[c];
+    const auto lo = S.ghost_node.begin() + S.ghost_begin[c], hi = S.ghost_node.begin() + S.ghost_begin[c + 1];
+    const auto at = std::lower_bound(lo, hi, node);
+    if (at == hi || *at != node) return 0;  // direct schedules: read in place
+    return S.patch_begin[c + 1] - S.patch_begin[c] + static_cast<uint32_t>(at - lo);
+}
+
+// Records of every kind in schedule order.
+static void emit_records(const OwnedDefinition& d, ClusterSchedule& S,
+                         const std::array<std::vector<std::array<uint32_t, 4>>, 3>& kind_nodes,
+                         const std::array<std::vector<int>, 3>& kind_counts,
+                         const std::array<std::vector<int>, 3>& kind_cta,
+                         const std::array<std::vector<int>, 3>& kind_colour, bool direct) {
+    const int ctas = S.ctas;
+    // a boundary node: its home and every CTA that touches it are not one
+    std::vector<int> home(S.node_count);
+    std::vector<uint8_t> shared(S.node_count, 0);
+    for (int c = 0; c < ctas; ++c)
+        for (uint32_t s = S.patch_begin[c]; s < S.patch_begin[c + 1]; ++s) home[S.node_of_slot[s]] = c;
+    for (int k = 0; k < 3; ++k)
+        for (size_t i = 0; i < kind_counts[k].size(); ++i)
+            for (int q = 0; q < kind_counts[k][i]; ++q)
+                if (home[kind_nodes[k][i][q]] != kind_cta[k][i]) shared[kind_nodes[k][i][q]] = 1;
+    for (int k = 0; k < 3; ++k) {
+        ClusterKind& K = S.kinds[k];
+        const auto& nodes = kind_nodes[k];
+        const auto& counts = kind_counts[k];
+        const auto& cta_of = kind_cta[k];
+        const auto& colour = kind_colour[k];
+        const size_t m = counts.size();
+        const int stages = K.stages;
+        std::vector<uint8_t> edge(m, 0);
+        for (size_t i = 0; i < m; ++i)
+            for (int q = 0; q < counts[i]; ++q)
+                // in a direct schedule only the records with foreign nodes
+                edge[i] |= direct ? home[nodes[i][q]] != cta_of[i] : shared[nodes[i][q]] != 0;
+        // CTA-major, stage within, boundary records first, definition order within
+        std::vector<uint32_t> idx(m);
+        std::iota(idx.begin(), idx.end(), 0u);
+        std::stable_sort(idx.begin(), idx.end(), [&](uint32_t x, uint32_t y) {
+            if (cta_of[x] != cta_of[y]) return cta_of[x] < cta_of[y];
+            if (colour[x] != colour[y]) return colour[x] < colour[y];
+            return edge[x] > edge[y];
+        });
+        K.offsets.assign(static_cast<size_t>(ctas) * (stages + 1), 0);
+        K.boundary.assign(static_cast<size_t>(ctas) * stages, 0);
+        K.boundary_first.assign(static_cast<size_t>(ctas) * stages, 0);
+        std::vector<uint32_t> count(static_cast<size_t>(ctas) * std::max(stages, 1), 0);
+        for (size_t i = 0; i < m; ++i) {
+            ++count[static_cast<size_t>(cta_of[i]) * stages + colour[i]];
+            K.boundary[static_cast<size_t>(cta_of[i]) * stages + colour[i]] += edge[i];
+        }
+        K.max_cta_records = 0;
+        K.boundary_total = 0;
+        uint32_t off = 0;
+        for (int c = 0; c < ctas; ++c) {
+            const uint32_t cta_start = off;
+            for (int s = 0; s < stages; ++s) {
+                K.offsets[static_cast<size_t>(c) * (stages + 1) + s] = off;
+                off += count[static_cast<size_t>(c) * stages + s];
+                K.boundary_first[static_cast<size_t>(c) * stages + s] = K.boundary_total;
+                K.boundary_total += K.boundary[static_cast<size_t>(c) * stages + s];
+            }
+            K.offsets[static_cast<size_t>(c) * (stages + 1) + stages] = off;
+            K.max_cta_records = std::max(K.max_cta_records, off - cta_start);
+        }
+        for (auto* v : {&K.ab, &K.cd, &K.lab, &K.lcd, &K.def_index}) v->clear();
+        K.rest.clear();
+        K.comp.clear();
+        for (uint32_t i : idx) {
+            const int c = cta_of[i];
+            K.ab.push_back(make_ref(S, nodes[i][0]) | (make_ref(S, nodes[i][1]) << 16));
+            K.lab.push_back(local_slot(S, c, nodes[i][0]) | (local_slot(S, c, nodes[i][1]) << 16));
+            if (k == 2) {
+                K.cd.push_back(make_ref(S, nodes[i][2]));
+                K.lcd.push_back(local_slot(S, c, nodes[i][2]));
+                K.rest.push_back(0.0f);
+                K.comp.push_back(0.0f);
+            } else if (k == 1) {
+                K.cd.push_back(make_ref(S, nodes[i][2]) | (make_ref(S, nodes[i][3]) << 16));
+                K.lcd.push_back(local_slot(S, c, nodes[i][2]) | (local_slot(S, c, nodes[i][3]) << 16));
+                K.rest.push_back(static_cast<float>(d.dihedrals[i].rest_angle));
+                K.comp.push_back(static_cast<float>(d.dihedrals[i].compliance));
+            } else {
+                const auto& dc = d.constraints[i];
+                const bool stitch = dc.kind == SWB_CONSTRAINT_SEAM_STITCH;
+                K.lcd.push_back(0);
+                K.rest.push_back(stitch ? 0.0f : static_cast<float>(dc.rest_length));
+                float cp = stitch ? 0.0f : static_cast<float>(dc.compliance);
+                if (dc.kind == SWB_CONSTRAINT_CABLE) cp = std::copysign(std::fabs(cp), -1.0f);
+                K.comp.push_back(cp);
+            }
+            K.def_index.push_back(i);
+        }
+    }
+}
+
+ClusterFlow build_flow(const OwnedDefinition& d, const ClusterSchedule& S, bool reverse, bool direct) {
+    const int C = S.ctas, G = total_stages(S);
+    ClusterFlow F;
+    F.direct = direct;
+    for (int k = 0; k < 3; ++k) F.send[k].assign(S.kinds[k].boundary_total, {0, 0, 0, 0});
+    F.barrier.assign(static_cast<size_t>(C) * G, 0);
+    F.out_begin.assign(C + 1, 0);
+    F.bytes_begin.assign(C + 1, 0);
+    std::vector<int> home(S.node_count);
+    for (int c = 0; c < C; ++c)
+        for (uint32_t s = S.patch_begin[c]; s < S.patch_begin[c + 1]; ++s) home[S.node_of_slot[s]] = c;
+    std::vector<std::vector<uint32_t>> bytes(C, std::vector<uint32_t>(1, 0));
+    auto receive = [&](int c, int g) {  // the barrier of CTA c's stage g, one more node on it
+        uint32_t& b = F.barrier[static_cast<size_t>(c) * G + g];
+        if (b == 0) {
+            b = static_cast<uint32_t>(bytes[c].size());
+            bytes[c].push_back(0);
+        }
+        bytes[c][b] += 16;
+        return b;
+    };
+    // each boundary node's last touch so far: CTA and its send word
+    struct Touch { int cta = -1; uint32_t* word = nullptr; };
+    std::vector<Touch> last(S.node_count);
+    std::vector<std::vector<std::array<uint32_t, 2>>> out(C);
+    for (int step = 0; step < G; ++step) {
+        const int g = reverse ? G - 1 - step : step;
+        int k, s;
+        global_stage(S, g, k, s);
+        const ClusterKind& K = S.kinds[k];
+        for (int c = 0; c < C; ++c) {
+            const uint32_t lo = K.offsets[static_cast<size_t>(c) * (K.stages + 1) + s];
+            const size_t cs = static_cast<size_t>(c) * K.stages + s;
+            for (uint32_t j = 0; j < K.boundary[cs]; ++j) {
+                uint32_t nodes[4];
+                const int cnt = element_nodes(d, k, K.def_index[lo + j], nodes);
+                std::array<uint32_t, 4>& words = F.send[k][K.boundary_first[cs] + j];
+                for (int q = 0; q < cnt; ++q) {
+                    const uint32_t n = nodes[q];
+                    if (direct) {
+                        if (home[n] != c)
+                            words[q] = send_word(static_cast<uint32_t>(home[n]), 0,
+                                                 S.slot_of_node[n] - S.patch_begin[home[n]]);
+                        continue;
+                    }
+                    Touch& t = last[n];
+                    if (t.cta < 0) {
+                        if (home[n] != c)
+                            out[home[n]].push_back({local_slot(S, home[n], n),
+                                                    send_word(static_cast<uint32_t>(c), receive(c, g),
+                                                              local_slot(S, c, n))});
+                    } else if (t.cta != c) {
+                        *t.word = send_word(static_cast<uint32_t>(c), receive(c, g), local_slot(S, c, n));
+                    }
+                    t = {c, &words[q]};
+                }
+            }
+        }
+    }
+    for (uint32_t n = 0; n < S.node_count; ++n)
+        if (last[n].cta >= 0 && last[n].cta != home[n]) {
+            bytes[home[n]][0] += 16;
+            *last[n].word = send_word(static_cast<uint32_t>(home[n]), 0, local_slot(S, home[n], n));
+        }
+    for (int c = 0; c < C; ++c) {
+        F.out.insert(F.out.end(), out[c].begin(), out[c].end());
+        F.out_begin[c + 1] = static_cast<uint32_t>(F.out.size());
+        F.bytes.insert(F.bytes.end(), bytes[c].begin(), bytes[c].end());
+        F.bytes_begin[c + 1] = static_cast<uint32_t>(F.bytes.size());
+        F.max_barriers = std::max(F.max_barriers, static_cast<uint32_t>(bytes[c].size()));
+    }
+    return F;
+}
+
+std::vector<std::array<uint32_t, 4>> stage_descriptors(const ClusterSchedule& S, const ClusterFlow& F) {
+    const int G = total_stages(S);
+    std::vector<std::array<uint32_t, 4>> out(static_cast<size_t>(S.ctas) * G);
+    uint32_t record_first[3] = {0, 0, 0}, send_first[3] = {0, 0, 0};
+    for (int k = 1; k < 3; ++k) {
+        record_first[k] = record_first[k - 1] + static_cast<uint32_t>(S.kinds[k - 1].ab.size());
+        send_first[k] = send_first[k - 1] + S.kinds[k - 1].boundary_total;
+    }
+    for (int c = 0; c < S.ctas; ++c)
+        for (int g = 0; g < G; ++g) {
+            int k, s;
+            global_stage(S, g, k, s);
+            const ClusterKind& K = S.kinds[k];
+            const size_t o = static_cast<size_t>(c) * (K.stages + 1), cs = static_cast<size_t>(c) * K.stages + s;
+            out[static_cast<size_t>(c) * G + g] = {record_first[k] + K.offsets[o + s],
+                                                   K.offsets[o + s + 1] - K.offsets[o + s],
+                                                   send_first[k] + K.boundary_first[cs],
+                                                   K.boundary[cs] | F.barrier[static_cast<size_t>(c) * G + g] << 16};
+        }
+    return out;
+}
+
+ClusterLayout layout_of(const ClusterSchedule& s) {
+    auto align = [](uint64_t v) { return (v + 15) & ~uint64_t{15}; };
+    ClusterLayout L;
+    uint64_t off = align(s.max_local * 16ull);
+    L.velocity = static_cast<uint32_t>(off);
+    uint64_t lam = off;
+    for (int k = 0; k < 3; ++k) {
+        L.lambda[k] = static_cast<uint32_t>(lam);
+        lam = align(lam + s.kinds[k].max_cta_records * (k == 2 ? 12ull : 4ull));
+    }
+    off = std::max(lam, align(off + s.max_patch * 16ull));
+    L.stages = kStagesInGlobal;
+    if (total_stages(s) <= kSharedStages) {
+        L.stages = static_cast<uint32_t>(off);
+        off = align(off + total_stages(s) * 16ull);
+    }
+    L.barriers = static_cast<uint32_t>(off);
+    if (!s.forward.direct) off = align(off + s.forward.max_barriers * 8ull);
+    L.bytes = static_cast<uint32_t>(off);
+    if (!s.forward.direct) off = align(off + s.forward.max_barriers * 4ull);
+    L.total = static_cast<uint32_t>(std::min<uint64_t>(off, 0xffffffffu));
+    return L;
+}
+
 bool build_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_t>& suspension_nodes, int ctas,
-                            ClusterSchedule& S, bool split) {
+                            ClusterSchedule& S, bool split, size_t shared_limit) {
     S = ClusterSchedule{};
     const uint32_t N = static_cast<uint32_t>(d.nodes.size());
     ctas = std::clamp(ctas, 1, kClusterMaxCtas);
@@ -334,39 +625,36 @@ bool build_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_t
     S.ctas = ctas;
     S.node_count = N;
     const std::vector<int> part = bisect_nodes(d, suspension_nodes, ctas, 0.03);
-    S.patch_begin.assign(ctas + 1, 0);
-    for (uint32_t n = 0; n < N; ++n) ++S.patch_begin[part[n] + 1];
-    for (int c = 0; c < ctas; ++c) {
-        S.max_patch = std::max(S.max_patch, S.patch_begin[c + 1]);
-        S.patch_begin[c + 1] += S.patch_begin[c];
-    }
-    if (S.max_patch > kClusterPatchNodes) {
-        S = ClusterSchedule{};
-        return false;
-    }
-    S.node_of_slot.assign(N, 0);
-    S.slot_of_node.assign(N, 0);
     {
-        std::vector<uint32_t> cur(S.patch_begin.begin(), S.patch_begin.end() - 1);
-        for (uint32_t n = 0; n < N; ++n) {
-            const uint32_t s = cur[part[n]]++;
-            S.node_of_slot[s] = n;
-            S.slot_of_node[n] = s;
+        std::vector<uint32_t> size(ctas, 0);
+        for (uint32_t n = 0; n < N; ++n) ++size[part[n]];
+        S.max_part = *std::max_element(size.begin(), size.end());
+        if (S.max_part > kClusterPatchNodes) {
+            S = ClusterSchedule{};
+            return false;
         }
     }
+    std::vector<uint8_t> attached(N, 0);
+    for (uint32_t n : suspension_nodes) attached[n] = 1;
     if (!suspension_nodes.empty()) S.susp_cta = part[suspension_nodes[0]];
 
+    // per kind: nodes, executing CTA and stage of every element
+    std::array<std::vector<std::array<uint32_t, 4>>, 3> kind_nodes;
+    std::array<std::vector<int>, 3> kind_counts, kind_cta, kind_colour;
     for (int k = 0; k < 3; ++k) {
         ClusterKind& K = S.kinds[k];
         const size_t m = k == 0 ? d.constraints.size() : (k == 1 ? d.dihedrals.size() : d.membranes.size());
-        std::vector<std::array<uint32_t, 4>> nodes(m);
-        std::vector<int> counts(m, 0);
+        std::vector<std::array<uint32_t, 4>>& nodes = kind_nodes[k];
+        std::vector<int>& counts = kind_counts[k];
+        nodes.resize(m);
+        counts.assign(m, 0);
         for (size_t i = 0; i < m; ++i) {
             nodes[i] = {0, 0, 0, 0};
             counts[i] = element_nodes(d, k, i, nodes[i].data());
         }
         // executing CTA: owner of most of the constraint's nodes (ties: first)
-        std::vector<int> cta_of(m, 0);
+        std::vector<int>& cta_of = kind_cta[k];
+        cta_of.assign(m, 0);
         std::vector<uint8_t> interior(m, 0);
         for (size_t i = 0; i < m; ++i) {
             int best = part[nodes[i][0]], best_count = 0;
@@ -381,7 +669,8 @@ bool build_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_t
             cta_of[i] = best;
             interior[i] = best_count == counts[i];
         }
-        std::vector<int> colour(m, 0);  // becomes the stage
+        std::vector<int>& colour = kind_colour[k];  // becomes the stage
+        colour.assign(m, 0);
         if (!split || ctas == 1 || k == 2) {  // membranes: classic stages
             K.stages = dsatur_colour(nodes, counts, colour);
             K.stages = reduce_colours(nodes, counts, N, K.stages, colour, kColourSearchMoves);
@@ -463,64 +752,49 @@ bool build_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_t
             K.cluster_sync.assign(K.stages, 1);
             for (int g = 0; g + 1 < inner_only; ++g) K.cluster_sync[g] = 0;
         }
-        const int stages = K.stages;
-        // records CTA-major, stage within, definition order within
-        std::vector<uint32_t> idx(m);
-        std::iota(idx.begin(), idx.end(), 0u);
-        std::stable_sort(idx.begin(), idx.end(), [&](uint32_t x, uint32_t y) {
-            if (cta_of[x] != cta_of[y]) return cta_of[x] < cta_of[y];
-            return colour[x] < colour[y];
-        });
-        K.offsets.assign(static_cast<size_t>(ctas) * (stages + 1), 0);
-        std::vector<uint32_t> count(static_cast<size_t>(ctas) * std::max(stages, 1), 0);
-        for (size_t i = 0; i < m; ++i) ++count[static_cast<size_t>(cta_of[i]) * stages + colour[i]];
-        uint32_t off = 0;
-        for (int c = 0; c < ctas; ++c) {
-            const uint32_t cta_start = off;
-            for (int s = 0; s < stages; ++s) {
-                K.offsets[static_cast<size_t>(c) * (stages + 1) + s] = off;
-                off += count[static_cast<size_t>(c) * stages + s];
-            }
-            K.offsets[static_cast<size_t>(c) * (stages + 1) + stages] = off;
-            K.max_cta_records = std::max(K.max_cta_records, off - cta_start);
-        }
-        for (uint32_t i : idx) {
-            K.ab.push_back(make_ref(S, nodes[i][0]) | (make_ref(S, nodes[i][1]) << 16));
-            if (k == 2) {
-                K.cd.push_back(make_ref(S, nodes[i][2]));
-                K.rest.push_back(0.0f);
-                K.comp.push_back(0.0f);
-            } else if (k == 1) {
-                K.cd.push_back(make_ref(S, nodes[i][2]) | (make_ref(S, nodes[i][3]) << 16));
-                K.rest.push_back(static_cast<float>(d.dihedrals[i].rest_angle));
-                K.comp.push_back(static_cast<float>(d.dihedrals[i].compliance));
-            } else {
-                const auto& dc = d.constraints[i];
-                const bool stitch = dc.kind == SWB_CONSTRAINT_SEAM_STITCH;
-                K.rest.push_back(stitch ? 0.0f : static_cast<float>(dc.rest_length));
-                float cp = stitch ? 0.0f : static_cast<float>(dc.compliance);
-                if (dc.kind == SWB_CONSTRAINT_CABLE) cp = std::copysign(std::fabs(cp), -1.0f);
-                K.comp.push_back(cp);
-            }
-            K.def_index.push_back(i);
-        }
-        // sweep order: stage-major, CTA, record order
+        // sweep order: stage-major, CTA of the bisection, definition order
         auto& order = k == 0 ? S.distance_order : (k == 1 ? S.dihedral_order : S.membrane_order);
-        for (int s = 0; s < stages; ++s)
-            for (int c = 0; c < ctas; ++c)
-                for (uint32_t r = K.offsets[static_cast<size_t>(c) * (stages + 1) + s];
-                     r < K.offsets[static_cast<size_t>(c) * (stages + 1) + s + 1]; ++r)
-                    order.push_back(K.def_index[r]);
+        order.resize(m);
+        std::iota(order.begin(), order.end(), uint64_t{0});
+        std::stable_sort(order.begin(), order.end(), [&](uint64_t x, uint64_t y) {
+            if (colour[x] != colour[y]) return colour[x] < colour[y];
+            return cta_of[x] < cta_of[y];
+        });
+        // the suspension nodes are the suspension CTA's alone: the line
+        // iteration works on its shared memory
+        for (size_t i = 0; i < m; ++i)
+            for (int q = 0; q < counts[i]; ++q)
+                if (attached[nodes[i][q]]) cta_of[i] = S.susp_cta;
+    }
+
+    // Patches may outgrow the bisection's parts by the homes they take, as far
+    // as the reverse sweep of a rollout (nodes, their start adjoints, three
+    // values per distance record, two per dihedral) keeps its room.
+    uint64_t records[2] = {0, 0};
+    for (int k = 0; k < 2; ++k) {
+        std::vector<uint64_t> count(ctas, 0);
+        for (int c : kind_cta[k]) ++count[c];
+        records[k] = *std::max_element(count.begin(), count.end());
+    }
+    const uint64_t reverse = 32ull * S.max_part + 12 * records[0] + 8 * records[1] + 4ull * (total_stages(S) + 2) + 112;
+    const uint64_t room = reverse < shared_limit ? (shared_limit - reverse) / 32 : 0;
+    const uint32_t patch_limit = static_cast<uint32_t>(std::min<uint64_t>(kClusterPatchNodes, S.max_part + room));
+    bool direct = false;
+    for (;;) {
+        place_nodes(S, part, kind_nodes, kind_counts, kind_cta, kind_colour, attached, patch_limit, direct);
+        emit_records(d, S, kind_nodes, kind_counts, kind_cta, kind_colour, direct);
+        S.forward = build_flow(d, S, false, direct);
+        if (direct || (S.max_local <= kSendSlots && S.forward.max_barriers <= kSendBarriers &&
+                       layout_of(S).total <= shared_limit))
+            break;
+        direct = true;
     }
 
     // line iteration window: the last two stages of the iteration, when
-    // neither touches a suspension endpoint node (classic stages: both end in
-    // a cluster barrier)
+    // neither touches a suspension endpoint node
     if (S.susp_cta >= 0 && !(split && ctas > 1)) {
-        std::vector<uint8_t> attached(N, 0);
-        for (uint32_t n : suspension_nodes) attached[n] = 1;
         const int Sg = total_stages(S);
-        if (Sg >= 2 && !stage_touches(d, S, attached, Sg - 2) && !stage_touches(d, S, attached, Sg - 1)) {
+        if (Sg >= 2 && !direct && !stage_touches(d, S, attached, Sg - 2) && !stage_touches(d, S, attached, Sg - 1)) {
             S.line_stage = Sg - 2;
             for (int g = Sg - 2; g < Sg; ++g) {
                 int k, s;
@@ -545,7 +819,7 @@ bool build_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_t
             if (c.kind != SWB_CONSTRAINT_SEAM_STITCH) continue;
             const int s = std::max(node_stage[c.first_node], node_stage[c.second_node]) + 1;
             node_stage[c.first_node] = node_stage[c.second_node] = s;
-            recs.push_back({s, part[c.first_node], i});
+            recs.push_back({s, home_of(S, static_cast<uint32_t>(c.first_node)), i});
         }
         S.seam_stages = 0;
         for (const Rec& r : recs) S.seam_stages = std::max(S.seam_stages, r.stage + 1);
@@ -571,8 +845,87 @@ bool build_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_t
     return true;
 }
 
+// Checks a flow: walking the stages, every record finds each of its nodes in
+// its own CTA's array (or, in a direct schedule, marked with the node's
+// home), counted on the barrier its stage waits on; every node ends at home;
+// each barrier receives exactly the bytes it is armed with.
+void verify_flow(const OwnedDefinition& d, const ClusterSchedule& S, const ClusterFlow& F, bool reverse) {
+    auto fail = [](const std::string& what) { raise(SWB_INVALID_ARGUMENT, "cluster schedule hand-overs: " + what); };
+    const int C = S.ctas, G = total_stages(S);
+    std::vector<int> at(S.node_count);
+    std::vector<uint32_t> slot(S.node_count);
+    std::vector<int64_t> pending(S.node_count, -1);  // the barrier that counts the node's last send
+    std::vector<std::vector<uint32_t>> got(C);
+    for (int c = 0; c < C; ++c) got[c].assign(F.bytes_begin[c + 1] - F.bytes_begin[c], 0);
+    for (int c = 0; c < C; ++c)
+        for (uint32_t s = S.patch_begin[c]; s < S.patch_begin[c + 1]; ++s) {
+            at[S.node_of_slot[s]] = c;
+            slot[S.node_of_slot[s]] = s - S.patch_begin[c];
+        }
+    const std::vector<int> home = at;
+    auto node_at_local = [&](int c, uint32_t local) {
+        const uint32_t own = S.patch_begin[c + 1] - S.patch_begin[c];
+        if (local < own) return S.node_of_slot[S.patch_begin[c] + local];
+        if (local - own >= S.ghost_begin[c + 1] - S.ghost_begin[c]) fail("local reference past the ghosts");
+        return S.ghost_node[S.ghost_begin[c] + local - own];
+    };
+    auto send = [&](uint32_t n, uint32_t word) {
+        const int to = static_cast<int>(word >> 27 & 15u);
+        const uint32_t bar = word >> 14 & (kSendBarriers - 1), local = word & (kSendSlots - 1);
+        if (!(word & kSendValid) || to >= C || bar >= got[to].size()) fail("send word");
+        if (node_at_local(to, local) != n) fail("a send names another node's slot");
+        got[to][bar] += 16;
+        at[n] = to;
+        slot[n] = local;
+        pending[n] = bar;
+    };
+    for (int c = 0; c < C; ++c)
+        for (uint32_t e = F.out_begin[c]; e < F.out_begin[c + 1]; ++e) {
+            const uint32_t n = node_at_local(c, F.out[e][0]);
+            if (at[n] != c) fail("a node is sent out from a CTA that does not hold it");
+            send(n, F.out[e][1]);
+        }
+    for (int step = 0; step < G; ++step) {
+        const int g = reverse ? G - 1 - step : step;
+        int k, s;
+        global_stage(S, g, k, s);
+        const ClusterKind& K = S.kinds[k];
+        for (int c = 0; c < C; ++c) {
+            const size_t o = static_cast<size_t>(c) * (K.stages + 1) + s, cs = static_cast<size_t>(c) * K.stages + s;
+            const uint32_t barrier = F.barrier[static_cast<size_t>(c) * G + g];
+            for (uint32_t r = K.offsets[o]; r < K.offsets[o + 1]; ++r) {
+                uint32_t nodes[4];
+                const int cnt = element_nodes(d, k, K.def_index[r], nodes);
+                const bool edge = r - K.offsets[o] < K.boundary[cs];
+                const uint32_t local[4] = {K.lab[r] & 0xffffu, K.lab[r] >> 16, K.lcd[r] & 0xffffu, K.lcd[r] >> 16};
+                for (int q = 0; q < cnt; ++q) {
+                    const uint32_t n = nodes[q];
+                    const uint32_t word = edge ? F.send[k][K.boundary_first[cs] + (r - K.offsets[o])][q] : 0u;
+                    if (F.direct) {
+                        const uint32_t want = home[n] == c ? 0u : send_word(static_cast<uint32_t>(home[n]), 0, slot[n]);
+                        if (word != want || (!want && local[q] != slot[n])) fail("direct record's node");
+                        continue;
+                    }
+                    if (at[n] != c || slot[n] != local[q]) fail("a record's node is not in its CTA's array");
+                    if (pending[n] >= 0 && (!edge || pending[n] != static_cast<int64_t>(barrier) || barrier == 0))
+                        fail("a stage does not wait for a node it receives");
+                    pending[n] = -1;
+                    if (word) send(n, word);
+                }
+            }
+        }
+    }
+    if (F.direct) return;
+    for (uint32_t n = 0; n < S.node_count; ++n)
+        if (at[n] != home[n] || (pending[n] >= 0 && pending[n] != 0)) fail("a node does not come home");
+    for (int c = 0; c < C; ++c)
+        for (size_t b = 0; b < got[c].size(); ++b)
+            if (got[c][b] != F.bytes[F.bytes_begin[c] + b]) fail("bytes of a barrier");
+}
+
 void verify_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_t>& suspension_nodes,
                              const ClusterSchedule& S) {
+    verify_flow(d, S, S.forward, false);
     auto fail = [](const std::string& what) { raise(SWB_INVALID_ARGUMENT, "cluster schedule invariant: " + what); };
     const uint32_t N = static_cast<uint32_t>(d.nodes.size());
     const int C = S.ctas;

@@ -4,30 +4,45 @@
 // bisection, suspension endpoint nodes kept together) and live in that
 // CTA's shared memory for the whole step.  Each constraint kind is
 // coloured over the whole mesh (DSatur); a colour is one stage, and every
-// constraint of a stage is executed by the CTA that owns most of its nodes,
-// reaching nodes of other CTAs through distributed shared memory.  A
-// cluster barrier separates stages.  Node references are 16-bit: the owner
-// rank in the top 4 bits and the index in its patch in the low 12 bits.
+// constraint of a stage is executed by the CTA that owns most of its nodes
+// (the suspension CTA where it touches a suspension endpoint).
+//
+// Between stages a CTA waits only for itself (a CTA barrier): a node that
+// several CTAs touch is handed from one to the next.  Within an iteration a
+// node is touched by at most one record per stage, so its touches form a
+// sequence; where two touches in turn belong to different CTAs, the record
+// that finishes the first sends the node to the second CTA (a store into
+// its shared memory that counts on a barrier there, see cluster_kernel.cuh),
+// which waits for what its stage receives before the stage's boundary
+// records.  Every CTA keeps a copy slot (ghost) for each foreign node it
+// touches and reads its own shared memory only.  After its last touch of an
+// iteration a node returns home, to the CTA whose patch holds it: the first
+// to touch it in an iteration, so that the way home is also the way to its
+// next touch.  At the end of an iteration every node's value is at home,
+// where the passes between iterations (ground plane, contacts, seams) and
+// the kernel's epilogue find it.
+//
+// Direct flows (fallback, when the ghosts do not fit in shared memory: meshes
+// whose constraints join nodes at random over the patches): no ghosts; a
+// record reads and writes foreign nodes in place through distributed shared
+// memory, and a cluster barrier closes every stage.  A schedule's forward
+// sweep may hand over while its reverse, which needs more shared memory per
+// record, is direct.
+//
+// Node references are 16-bit: the home rank in the top 4 bits and the index
+// in its patch in the low 12 bits (home references), or the index in the
+// executing CTA's node array, ghosts after the patch (local references).
 //
 // Split stages (optional, SWB_OPT_SPLIT_STAGES): a constraint whose
 // nodes all lie in one CTA's patch is interior.  Per kind, the interior
-// constraints run first, coloured per CTA, with only a CTA barrier between
-// their stages (interior constraints of different CTAs share no node); one
-// cluster barrier follows.  The constraints that span CTAs are coloured
-// together; their large colours run one stage each with a cluster barrier
-// after it, and the short tail of small colours runs on a single CTA with CTA
-// barriers, closed by one cluster barrier.  Each stage carries the kind of
-// barrier that follows it.  Classic stages (the default: one colouring of
-// the whole mesh, a cluster barrier after every stage) are also what packed
-// batches need, whose structures must take identical barriers.  On the
-// B200 the classic form is faster: a stage's cost is mostly its records'
-// issue and latency, not its barrier, and split stages double the stages.
+// constraints run first, coloured per CTA; the constraints that span CTAs
+// are coloured together and their stages follow.
 //
-// Sweep order per kind: stage-major, then CTA rank, then record order --
-// the reference serial solver run on the definition permuted into this
+// Sweep order per kind: stage-major, then the CTA that owns most of a
+// constraint's nodes in the bisection, then definition order -- the
+// reference serial solver run on the definition permuted into this
 // order performs exactly the device sweep: constraints of one stage share
-// no node, and within a run of stages joined by CTA barriers every node is
-// touched by one CTA only.
+// no node, and every node meets its stages in order.
 #pragma once
 
 #include "common.h"
@@ -44,10 +59,16 @@ constexpr uint32_t kClusterPatchNodes = 4096;
 struct ClusterKind {
     int stages = 0;
     // [ctas * (stages + 1)]: record offsets of (cta, stage); records are
-    // stored CTA-major, stage within.
+    // stored CTA-major, stage within, boundary records first.
     std::vector<uint32_t> offsets;
-    std::vector<uint32_t> ab;    // ref(a) | ref(b) << 16
-    std::vector<uint32_t> cd;    // dihedral: ref(c) | ref(d) << 16
+    // [ctas * stages]: boundary records of (cta, stage), those that touch a
+    // node another CTA touches too, and the first of their entries in the
+    // flows' send tables (one entry per boundary record, in record order)
+    std::vector<uint32_t> boundary, boundary_first;
+    uint32_t boundary_total = 0;
+    std::vector<uint32_t> ab;    // home ref(a) | ref(b) << 16
+    std::vector<uint32_t> cd;    // dihedral: home ref(c) | ref(d) << 16
+    std::vector<uint32_t> lab, lcd;  // the same as local references
     std::vector<float> rest;
     std::vector<float> comp;     // distance: sign bit = cable
     std::vector<uint32_t> def_index;
@@ -58,12 +79,45 @@ struct ClusterKind {
     int interior_stages = 0, boundary_stages = 0;
 };
 
+// Where a record sends a node after its projection: 0 = nowhere (the node
+// stays in the executing CTA's array), else kSendValid | rank << 27 | the
+// barrier that counts it there << 14 | its slot in that CTA's node array.
+// In a direct flow the word marks a foreign node: its home rank and slot
+// (barrier 0), read and written in place.
+constexpr uint32_t kSendValid = 1u << 31;
+constexpr uint32_t kSendSlots = 1u << 14, kSendBarriers = 1u << 13;
+constexpr uint32_t send_word(uint32_t rank, uint32_t barrier, uint32_t slot) {
+    return kSendValid | rank << 27 | barrier << 14 | slot;
+}
+
+// The hand-overs of a sweep through the iteration's stages, forward or in
+// reverse.  Barriers are numbered per CTA: 0 counts the nodes that come home
+// at the end of an iteration, the others one receiving stage each.
+struct ClusterFlow {
+    bool direct = false;                  // foreign nodes in place, cluster barriers (see above)
+    std::array<std::vector<std::array<uint32_t, 4>>, 3> send;  // per kind, per boundary record, per node
+    std::vector<uint32_t> barrier;        // [ctas * stages]: the stage's barrier, 0 when it receives nothing
+    std::vector<uint32_t> bytes_begin;    // [ctas + 1] into bytes
+    std::vector<uint32_t> bytes;          // per barrier: bytes received per iteration
+    // nodes whose first touch of an iteration is not at home: the home CTA
+    // sends them out at the iteration's start ([ctas + 1] offsets; slot, word)
+    std::vector<uint32_t> out_begin;
+    std::vector<std::array<uint32_t, 2>> out;
+    uint32_t max_barriers = 0;            // per CTA
+};
+
 struct ClusterSchedule {
     int ctas = 0;
+    // [ctas + 1] into ghost_node: the foreign nodes a CTA touches, in the
+    // order of their slots after its patch; the largest patch with ghosts
+    std::vector<uint32_t> ghost_begin, ghost_node;
+    uint32_t max_local = 0;
+    ClusterFlow forward;
     uint32_t node_count = 0;
     std::vector<uint32_t> node_of_slot, slot_of_node;  // slots: patch-major
     std::vector<uint32_t> patch_begin;                 // [ctas + 1]
     uint32_t max_patch = 0;
+    uint32_t max_part = 0;                             // the bisection's largest part
     // kinds[0] distance-type constraints, kinds[1] dihedrals, kinds[2]
     // membrane elements; an iteration runs distance, membrane, then dihedral
     // stages (soft_body.cpp:1318-1369)
@@ -124,18 +178,46 @@ inline int cluster_barriers_per_iteration(const ClusterSchedule& s) {
     return n;
 }
 
-// Dynamic shared memory of the cluster step kernel for this schedule
-// (nodes, forces/velocities, multipliers -- three per membrane element --,
-// stage offsets; with slack for the 16-byte alignment of each array).
+// Shared memory a schedule is admitted by: nodes and velocities of the
+// bisection's largest part, every multiplier, stage offsets.  A schedule that
+// passes runs whatever its boundary is (a direct schedule takes no more).
 inline size_t cluster_shared_bytes(const ClusterSchedule& s) {
-    return s.max_patch * 32ull + s.kinds[0].max_cta_records * 4ull + s.kinds[1].max_cta_records * 4ull +
+    return s.max_part * 32ull + s.kinds[0].max_cta_records * 4ull + s.kinds[1].max_cta_records * 4ull +
            s.kinds[2].max_cta_records * 12ull + (total_stages(s) + 3) * 4ull + 80;
 }
 
+// Dynamic shared memory of the step kernel, byte offsets: the node array
+// (patch and ghosts) at 0; the multipliers, three per membrane element, and
+// in the same place, before and after the iterations, the patch's forces or
+// velocities; the stage descriptors (none above kSharedStages, read from
+// global memory then); the barriers and the bytes each receives.
+constexpr int kSharedStages = 256;
+constexpr uint32_t kStagesInGlobal = ~0u;  // ClusterFlowDev::smem_stages
+struct ClusterLayout {
+    uint32_t lambda[3] = {0, 0, 0};
+    uint32_t velocity = 0, stages = 0, barriers = 0, bytes = 0, total = 0;
+};
+ClusterLayout layout_of(const ClusterSchedule& s);
+
 // Returns false (and leaves `out` empty) when the mesh does not fit one
-// cluster of `ctas` CTAs (a patch over kClusterPatchNodes nodes).
+// cluster of `ctas` CTAs (a patch over kClusterPatchNodes nodes).  The
+// forward flow is direct when its layout with ghosts would exceed
+// `shared_limit` bytes.
 bool build_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_t>& suspension_nodes, int ctas,
-                            ClusterSchedule& out, bool split = false);
+                            ClusterSchedule& out, bool split = false, size_t shared_limit = 227 * 1024 - 6144);
+
+// The hand-overs of one sweep direction (see ClusterFlow).
+ClusterFlow build_flow(const OwnedDefinition& d, const ClusterSchedule& s, bool reverse, bool direct);
+
+// Checks a flow of a schedule; raises on failure (verify_cluster_schedule
+// checks the forward one).
+void verify_flow(const OwnedDefinition& d, const ClusterSchedule& s, const ClusterFlow& f, bool reverse);
+
+// Stage descriptors of a flow, [ctas * stages] (global stages): the first
+// record, the record count, the first boundary record's entry in the send
+// table, boundary records | barrier << 16.  Records and send entries of all
+// kinds are numbered together, kind after kind.
+std::vector<std::array<uint32_t, 4>> stage_descriptors(const ClusterSchedule& s, const ClusterFlow& f);
 
 // Move budget of the search for a colouring with fewer colours (per colour
 // count tried).

@@ -136,6 +136,19 @@ __device__ __forceinline__ void st_node(uint32_t addr, float4 v) {
                  : "memory");
 }
 
+// A node record of the CTA's own shared memory (volatile: in program order
+// with the barriers, which alone order other accesses).
+__device__ __forceinline__ float4 ld_own(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ void st_own(uint32_t addr, float4 v) {
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w));
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned int count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");

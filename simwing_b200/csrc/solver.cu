@@ -241,7 +241,9 @@ void StructureImpl::build(const swb_structure_definition& definition, const swb_
             for (; c <= kClusterMaxCtas; c *= 2) candidates.push_back(c);
         }
         for (int c : candidates) {
-            if (!build_cluster_schedule(def, susp_nodes, c, csched, (opt.flags & SWB_OPT_SPLIT_STAGES) != 0)) continue;
+            if (!build_cluster_schedule(def, susp_nodes, c, csched, (opt.flags & SWB_OPT_SPLIT_STAGES) != 0,
+                                        smem_limit))
+                continue;
             const size_t bytes = cluster_shared_bytes(csched);
             if (bytes > smem_limit) continue;
             cluster_mode = true;
@@ -256,7 +258,7 @@ void StructureImpl::build(const swb_structure_definition& definition, const swb_
         raise(SWB_UNSUPPORTED, "membrane elements need the cluster schedule (the mesh does not fit one)");
     if (!cluster_mode && def.has_contact)
         raise(SWB_UNSUPPORTED, "fabric self-contact needs the cluster schedule (the mesh does not fit one)");
-    uint32_t widest = 32;
+    uint32_t widest = 32, widest_single = 32;
     if (cluster_mode) {
         verify_cluster_schedule(def, susp_nodes, csched);
         G = csched.ctas;
@@ -264,12 +266,16 @@ void StructureImpl::build(const swb_structure_definition& definition, const swb_
         node_of_slot = csched.node_of_slot;
         susp_owner = csched.susp_cta;
         susp_base = susp_owner >= 0 ? csched.patch_begin[susp_owner] : 0;
-        for (int k = 0; k < 2; ++k) {
+        // a thread takes two distance-type records of a stage side by side
+        // (sweep_distance_pair), one dihedral or membrane element
+        for (int k = 0; k < 3; ++k) {
             const ClusterKind& K = csched.kinds[k];
             for (int c = 0; c < G; ++c)
                 for (int s = 0; s < K.stages; ++s) {
                     const size_t o = static_cast<size_t>(c) * (K.stages + 1) + s;
-                    widest = std::max(widest, K.offsets[o + 1] - K.offsets[o]);
+                    const uint32_t n = K.offsets[o + 1] - K.offsets[o];
+                    widest = std::max(widest, k == 0 ? (n + 1) / 2 : n);
+                    widest_single = std::max(widest_single, n);
                 }
         }
     } else {
@@ -299,7 +305,7 @@ void StructureImpl::build(const swb_structure_definition& definition, const swb_
     threads = opt.block_threads > 0
                   ? opt.block_threads
                   : static_cast<int>(std::clamp<uint32_t>((widest + 31) / 32 * 32, 64,
-                                                          cluster_mode ? dev::kClusterMaxThreads : 512));
+                                                          512));
     if (opt.block_threads <= 0 && cluster_mode && def.has_contact) threads = dev::kClusterMaxThreads;
     if (threads % 32 != 0 || threads < 32 || threads > (cluster_mode ? dev::kClusterMaxThreads : 1024))
         raise(SWB_INVALID_ARGUMENT, "block_threads out of range for the chosen schedule");
@@ -307,9 +313,11 @@ void StructureImpl::build(const swb_structure_definition& definition, const swb_
         // the line iteration needs a warp of the suspension CTA that is idle
         // in its two stages
         const int need = static_cast<int>((csched.line_owner_records + 31) / 32 * 32 + 32);
-        if (opt.block_threads <= 0 && need > threads && need <= dev::kClusterMaxThreads) threads = need;
+        if (opt.block_threads <= 0 && need > threads && need <= dev::kClusterThreads) threads = need;
         if (need > threads) csched.line_stage = -1;
     }
+    // the reverse sweep takes one record per thread
+    reverse_threads = std::max(threads, static_cast<int>(std::clamp<uint32_t>((widest_single + 31) / 32 * 32, 64, 512)));
 
     // ---- device images -------------------------------------------------------
     // The node states are FP32 offsets from an FP64 origin on a 1/256 m grid
@@ -375,6 +383,28 @@ static void membrane_constants(const swb_membrane_def& m, float4 out[kMembraneAu
     out[2] = make_float4(f(q.weft_pretension), f(cxx), f(cyy), f(czz));
     out[3] = make_float4(f(cxy), 0.0f, 0.0f, f(kxx));
     out[4] = make_float4(f(kyy), f(kzz), f(kxy), 0.0f);
+}
+
+ClusterFlowDev upload_flow(const ClusterSchedule& s, const ClusterFlow& f, std::vector<void*>& owned,
+                           cudaStream_t stream) {
+    auto quads = [&](const std::vector<std::array<uint32_t, 4>>& v) {
+        std::vector<uint4> q(v.size());
+        for (size_t i = 0; i < v.size(); ++i) q[i] = make_uint4(v[i][0], v[i][1], v[i][2], v[i][3]);
+        return dupload(owned, q, stream);
+    };
+    ClusterFlowDev F{};
+    F.stages = quads(stage_descriptors(s, f));
+    std::vector<std::array<uint32_t, 4>> send;
+    for (const auto& v : f.send) send.insert(send.end(), v.begin(), v.end());
+    F.send = quads(send);
+    F.bytes_begin = dupload(owned, f.bytes_begin, stream);
+    F.bytes = dupload(owned, f.bytes, stream);
+    F.out_begin = dupload(owned, f.out_begin, stream);
+    std::vector<uint2> out(f.out.size());
+    for (size_t i = 0; i < out.size(); ++i) out[i] = make_uint2(f.out[i][0], f.out[i][1]);
+    F.out = dupload(owned, out, stream);
+    F.direct = f.direct ? 1 : 0;
+    return F;
 }
 
 // One instance record per (input, output) buffer pair, so that a launch only
@@ -449,6 +479,8 @@ void StructureImpl::setup_line_contact() {
 void (*StructureImpl::step_kernel() const)(ClusterParams) {
     if (def.has_contact)
         return def.membranes.empty() ? dev::xpbd_cluster_contact_kernel : dev::xpbd_cluster_contact_membrane_kernel;
+    if (threads > dev::kClusterThreads)
+        return def.membranes.empty() ? dev::xpbd_cluster_kernel_wide : dev::xpbd_cluster_membrane_kernel_wide;
     return def.membranes.empty() ? dev::xpbd_cluster_kernel : dev::xpbd_cluster_membrane_kernel;
 }
 
@@ -586,42 +618,45 @@ void StructureImpl::upload_cluster_tables() {
     ClusterParams& cp = cparams;
     std::memset(&cp, 0, sizeof(cp));
     cp.ctas = G;
-    uint32_t off = 0;
-    cp.smem_x = off; off = align16(off + csched.max_patch * 16u);
-    cp.smem_v = off; off = align16(off + csched.max_patch * 16u);
+    const ClusterLayout layout = layout_of(csched);
     ClusterInstance base{};
     base.patch_begin = dupload(owned, csched.patch_begin, stream);
+    std::vector<uint4> records;
+    for (int k = 0; k < 3; ++k) {
+        const ClusterKind& K = csched.kinds[k];
+        base.record_first[k] = static_cast<uint32_t>(records.size());
+        for (size_t r = 0; r < K.lab.size(); ++r)
+            records.push_back(make_uint4(K.lab[r], K.lcd[r], std::bit_cast<uint32_t>(K.rest[r]),
+                                         std::bit_cast<uint32_t>(K.comp[r])));
+    }
+    base.records = dupload(owned, records, stream);
     for (int k = 0; k < 3; ++k) {
         const ClusterKind& K = csched.kinds[k];
         ClusterKindDev& dk = base.kind[k];
         dk.offsets = dupload(owned, K.offsets, stream);
-        std::vector<uint4> rec(K.ab.size());
-        for (size_t r = 0; r < rec.size(); ++r)
-            rec[r] = make_uint4(K.ab[r], k >= 1 ? K.cd[r] : 0u, std::bit_cast<uint32_t>(K.rest[r]),
-                                std::bit_cast<uint32_t>(K.comp[r]));
-        dk.rec = dupload(owned, rec, stream);
+        dk.rec = base.records + base.record_first[k];
+        std::vector<uint2> home(k == 0 && csched.pair_stages == 0 ? 0 : (k == 1 ? 0 : K.ab.size()));
+        for (size_t r = 0; r < home.size(); ++r) home[r] = make_uint2(K.ab[r], k == 2 ? K.cd[r] : 0u);
+        dk.home = dupload(owned, home, stream);
         if (k == 2) {
-            std::vector<float4> aux(rec.size() * kMembraneAux);
-            for (size_t r = 0; r < rec.size(); ++r) membrane_constants(def.membranes[K.def_index[r]], &aux[r * kMembraneAux]);
+            std::vector<float4> aux(K.ab.size() * kMembraneAux);
+            for (size_t r = 0; r < K.ab.size(); ++r) membrane_constants(def.membranes[K.def_index[r]], &aux[r * kMembraneAux]);
             dk.aux = dupload(owned, aux, stream);
             for (int b = 0; b < 3; ++b) {
-                d_mres[b] = dalloc<float>(owned, rec.size());
-                cuda_check(cudaMemsetAsync(d_mres[b], 0, std::max<size_t>(rec.size(), 1) * sizeof(float), stream),
+                d_mres[b] = dalloc<float>(owned, K.ab.size());
+                cuda_check(cudaMemsetAsync(d_mres[b], 0, std::max<size_t>(K.ab.size(), 1) * sizeof(float), stream),
                            "memset");
             }
         }
         dk.stages = K.stages;
-        dk.smem_lambda = off;
-        // stages from 64 on always take a cluster barrier (a superset of any CTA barrier)
-        dk.sync_mask = 0;
-        for (int g = 0; g < std::min(K.stages, 64); ++g)
-            if (K.cluster_sync[g]) dk.sync_mask |= 1ull << g;
-        dk.interior_stages = K.interior_stages;
-        off = align16(off + K.max_cta_records * (k == 2 ? 12u : 4u));
+        dk.smem_lambda = layout.lambda[k];
     }
-    cp.smem_offsets = off;
-    off = align16(off + (total_stages(csched) + 3) * 4u);
-    cluster_smem = off;
+    base.smem_v = layout.velocity;
+    base.flow = upload_flow(csched, csched.forward, owned, stream);
+    base.flow.smem_stages = layout.stages;
+    base.flow.smem_barriers = layout.barriers;
+    base.flow.smem_bytes = layout.bytes;
+    cluster_smem = layout.total;
     base.seam_offsets = dupload(owned, csched.seam_offsets, stream);
     base.seam_ab = dupload(owned, csched.seam_ab, stream);
     base.seam_stages = csched.seam_stages;
@@ -1050,6 +1085,11 @@ size_t dynamic_smem_limit(const cudaDeviceProp& prop) {
                           reinterpret_cast<const void*>(dev::xpbd_cluster_packed_kernel),
                           reinterpret_cast<const void*>(dev::xpbd_cluster_membrane_kernel),
                           reinterpret_cast<const void*>(dev::xpbd_cluster_packed_membrane_kernel),
+                          reinterpret_cast<const void*>(dev::xpbd_cluster_kernel_wide),
+                          reinterpret_cast<const void*>(dev::xpbd_cluster_packed_kernel_wide),
+                          reinterpret_cast<const void*>(dev::xpbd_cluster_membrane_kernel_wide),
+                          reinterpret_cast<const void*>(dev::xpbd_cluster_packed_membrane_kernel_wide),
+                          reinterpret_cast<const void*>(dev::xpbd_cluster_tape_kernel_wide),
                           reinterpret_cast<const void*>(dev::xpbd_cluster_contact_kernel),
                           reinterpret_cast<const void*>(dev::xpbd_cluster_contact_membrane_kernel),
                           reinterpret_cast<const void*>(dev::xpbd_cluster_tape_kernel),
@@ -1064,9 +1104,19 @@ size_t dynamic_smem_limit(const cudaDeviceProp& prop) {
     return prop.sharedMemPerBlockOptin > reserve ? prop.sharedMemPerBlockOptin - reserve : 0;
 }
 
-cudaError_t packed_kernel_limits(int max_dynamic_smem, bool non_portable_cluster) {
+namespace {
+
+using ClusterKernel = void (*)(ClusterParams);
+
+ClusterKernel packed_kernel(const cudaLaunchConfig_t& cfg, bool membranes) {
+    if (cfg.blockDim.x > static_cast<unsigned>(dev::kClusterThreads))
+        return membranes ? dev::xpbd_cluster_packed_membrane_kernel_wide : dev::xpbd_cluster_packed_kernel_wide;
+    return membranes ? dev::xpbd_cluster_packed_membrane_kernel : dev::xpbd_cluster_packed_kernel;
+}
+
+cudaError_t kernel_limits(std::initializer_list<ClusterKernel> kernels, int max_dynamic_smem, bool non_portable_cluster) {
     cudaError_t rc = cudaSuccess;
-    for (auto kernel : {dev::xpbd_cluster_packed_kernel, dev::xpbd_cluster_packed_membrane_kernel}) {
+    for (auto kernel : kernels) {
         if (rc == cudaSuccess)
             rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic_smem);
         if (rc == cudaSuccess && non_portable_cluster)
@@ -1075,30 +1125,36 @@ cudaError_t packed_kernel_limits(int max_dynamic_smem, bool non_portable_cluster
     return rc;
 }
 
+}  // namespace
+
+cudaError_t packed_kernel_limits(int max_dynamic_smem, bool non_portable_cluster) {
+    return kernel_limits({dev::xpbd_cluster_packed_kernel, dev::xpbd_cluster_packed_membrane_kernel,
+                          dev::xpbd_cluster_packed_kernel_wide, dev::xpbd_cluster_packed_membrane_kernel_wide},
+                         max_dynamic_smem, non_portable_cluster);
+}
+
 cudaError_t packed_kernel_occupancy(int* clusters, const cudaLaunchConfig_t& cfg, bool membranes) {
-    return cudaOccupancyMaxActiveClusters(
-        clusters, membranes ? dev::xpbd_cluster_packed_membrane_kernel : dev::xpbd_cluster_packed_kernel, &cfg);
+    return cudaOccupancyMaxActiveClusters(clusters, packed_kernel(cfg, membranes), &cfg);
 }
 
 cudaError_t packed_kernel_launch(const cudaLaunchConfig_t& cfg, const ClusterParams& params, bool membranes) {
-    return cudaLaunchKernelEx(
-        &cfg, membranes ? dev::xpbd_cluster_packed_membrane_kernel : dev::xpbd_cluster_packed_kernel, params);
+    return cudaLaunchKernelEx(&cfg, packed_kernel(cfg, membranes), params);
 }
 
 cudaError_t plain_cluster_launch(const cudaLaunchConfig_t& cfg, const ClusterParams& params) {
-    return cudaLaunchKernelEx(&cfg, dev::xpbd_cluster_kernel, params);
+    return cudaLaunchKernelEx(
+        &cfg, cfg.blockDim.x > dev::kClusterThreads ? dev::xpbd_cluster_kernel_wide : dev::xpbd_cluster_kernel, params);
 }
 
 cudaError_t tape_kernel_limits(int max_dynamic_smem, bool non_portable_cluster) {
-    cudaError_t rc = cudaFuncSetAttribute(dev::xpbd_cluster_tape_kernel,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic_smem);
-    if (rc == cudaSuccess && non_portable_cluster)
-        rc = cudaFuncSetAttribute(dev::xpbd_cluster_tape_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    return rc;
+    return kernel_limits({dev::xpbd_cluster_tape_kernel, dev::xpbd_cluster_tape_kernel_wide}, max_dynamic_smem,
+                         non_portable_cluster);
 }
 
 cudaError_t tape_kernel_launch(const cudaLaunchConfig_t& cfg, const ClusterParams& params) {
-    return cudaLaunchKernelEx(&cfg, dev::xpbd_cluster_tape_kernel, params);
+    return cudaLaunchKernelEx(
+        &cfg, cfg.blockDim.x > dev::kClusterThreads ? dev::xpbd_cluster_tape_kernel_wide : dev::xpbd_cluster_tape_kernel,
+        params);
 }
 
 cudaError_t adjoint_kernel_limits(int max_dynamic_smem, bool non_portable_cluster) {

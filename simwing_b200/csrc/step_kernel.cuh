@@ -37,46 +37,101 @@ __device__ __forceinline__ float wrap_two_pi(float x) {
     return remainderf(x, kTwoPiF);
 }
 
+// The projections state each multiply-add themselves (__fmaf_rn, __fmul_rn,
+// __fadd_rn): the compiler's choice of which product of a sum to fuse depends
+// on the code around it, and every kernel must round alike.  They run
+// straight through, without early returns: a warp's records nearly always
+// take the full path, and the branches around it cost more than it does.
+__device__ __forceinline__ float fma_dot(float3 a, float3 b) {
+    return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+}
+__device__ __forceinline__ float3 fma_cross(float3 a, float3 b) {
+    return make_float3(__fmaf_rn(a.y, b.z, -__fmul_rn(a.z, b.y)), __fmaf_rn(a.z, b.x, -__fmul_rn(a.x, b.z)),
+                       __fmaf_rn(a.x, b.y, -__fmul_rn(a.y, b.x)));
+}
+__device__ __forceinline__ float3 rn_sub(float3 a, float3 b) {
+    return make_float3(__fadd_rn(a.x, -b.x), __fadd_rn(a.y, -b.y), __fadd_rn(a.z, -b.z));
+}
+__device__ __forceinline__ float3 rn_add(float3 a, float3 b) {
+    return make_float3(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z));
+}
+__device__ __forceinline__ float3 rn_scale(float3 a, float s) {
+    return make_float3(__fmul_rn(a.x, s), __fmul_rn(a.y, s), __fmul_rn(a.z, s));
+}
+__device__ __forceinline__ void fma_add(float4& p, float s, float3 d) {  // p += s d
+    p.x = __fmaf_rn(s, d.x, p.x);
+    p.y = __fmaf_rn(s, d.y, p.y);
+    p.z = __fmaf_rn(s, d.z, p.z);
+}
+// 1 / sqrt(x) of a positive normal number.
+__device__ __forceinline__ float rsqrt_normal(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+// fast_rcp (fast_math.h) without the scaling of arguments outside the
+// normal range: the same bits for 2^-126 <= |x| <= 2^126.
+__device__ __forceinline__ float rcp_normal(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // projectDistanceConstraint (soft_body.cpp:1598-1640) on float4 nodes
 // (xyz, w = inverse mass).  comp carries the cable flag in its sign bit.
 // The length and the two divisions use the reciprocal square root and the
 // approximate reciprocal (an ulp or two each) instead of IEEE sqrt and
-// division.
-__device__ __forceinline__ void project_distance(float4& pa, float4& pb, float rest, float comp_raw,
+// division.  False when the reference leaves the constraint alone; the nodes
+// and the multiplier are then not to be stored.
+__device__ __forceinline__ bool project_distance(float4& pa, float4& pb, float rest, float comp_raw,
                                                  float& lambda, float inv_dt2) {
-    const float dx = pb.x - pa.x, dy = pb.y - pa.y, dz = pb.z - pa.z;
-    const float l2 = dx * dx + dy * dy + dz * dz;
-    if (!(l2 > kMinimumLengthF * kMinimumLengthF)) return;
-    const float il = rsqrtf(l2);
-    const float l = l2 * il;
-    if (l <= kMinimumLengthF) return;
-    const float value = l - rest;
+    const float3 d = rn_sub(f3(pb), f3(pa));
+    const float l2 = fma_dot(d, d);
+    const float il = rsqrt_normal(l2);
+    const float l = __fmul_rn(l2, il);
+    const float value = __fadd_rn(l, -rest);
     const bool cable = signbit(comp_raw);
-    if (cable && value <= 0.0f && lambda == 0.0f) return;
-    const float wsum = pa.w + pb.w;
-    const float alpha = fabsf(comp_raw) * inv_dt2;
-    if (wsum + alpha <= 0.0f) return;
-    const float dl = (-value - alpha * lambda) * fast_rcp(wsum + alpha);
-    float applied = dl;
-    if (cable) {
-        const float sum = lambda + dl;
-        const float nl = sum < 0.0f ? sum : 0.0f;  // std::min(0.0, x)
-        applied = nl - lambda;
-        lambda = nl;
-    } else {
-        lambda += dl;
-    }
-    const float scale = applied * il;
-    const float sa = pa.w * scale, sb = pb.w * scale;
-    pa.x -= sa * dx; pa.y -= sa * dy; pa.z -= sa * dz;
-    pb.x += sb * dx; pb.y += sb * dy; pb.z += sb * dz;
+    const float wsum = __fadd_rn(pa.w, pb.w);
+    const float alpha = __fmul_rn(fabsf(comp_raw), inv_dt2);
+    const float den = __fadd_rn(wsum, alpha);
+    const bool ok = l2 > kMinimumLengthF * kMinimumLengthF && !(l <= kMinimumLengthF) &&
+                    !(cable && value <= 0.0f && lambda == 0.0f) && !(den <= 0.0f);
+    const float dl = __fmul_rn(__fmaf_rn(-alpha, lambda, -value), rcp_normal(den));
+    const float sum = __fadd_rn(lambda, dl);
+    const float nl = cable ? (sum < 0.0f ? sum : 0.0f) : sum;  // std::min(0.0, x)
+    const float applied = cable ? __fadd_rn(nl, -lambda) : dl;
+    lambda = nl;
+    const float scale = __fmul_rn(applied, il);
+    fma_add(pa, -__fmul_rn(pa.w, scale), d);
+    fma_add(pb, __fmul_rn(pb.w, scale), d);
+    return ok;
+}
+
+// fast_atan2 (fast_math.h) of a pair that is not NaN, without its branches.
+__device__ __forceinline__ float atan2_straight(float y, float x) {
+    const float ax = fabsf(x), ay = fabsf(y);
+    const float mx = fmaxf(ax, ay), mn = fminf(ax, ay);
+    const float a = __fmul_rn(mn, rcp_normal(mx));
+    const float s = __fmul_rn(a, a);
+    float p = -0.0043553877621889114f;
+    p = __fmaf_rn(p, s, 0.023040074855089188f);
+    p = __fmaf_rn(p, s, -0.05777350813150406f);
+    p = __fmaf_rn(p, s, 0.0979422926902771f);
+    p = __fmaf_rn(p, s, -0.13976579904556274f);
+    p = __fmaf_rn(p, s, 0.19962704181671143f);
+    p = __fmaf_rn(p, s, -0.3333165943622589f);
+    float r = __fmaf_rn(__fmul_rn(a, s), p, a);
+    r = ay > ax ? __fadd_rn(1.57079632679489662f, -r) : r;
+    r = mx > 0.0f ? r : 0.0f;
+    r = x < 0.0f ? __fadd_rn(3.14159265358979324f, -r) : r;
+    return copysignf(r, y);
 }
 
 // evaluateDihedral + solveDihedralConstraint (soft_body.cpp:1648-1711,
 // 1754-1792): one XPBD projection of the signed hinge angle.
 //
-// The angle uses fast_atan2 (fast_math.h, within 4e-7 rad of atan2) and the
-// divisions the approximate reciprocal.
+// The angle uses fast_atan2's arithmetic (fast_math.h, within 4e-7 rad of
+// atan2) and the divisions the approximate reciprocal.
 // The reference evaluates theta = atan2(e.(n1 x n2), n1.n2) from unit
 // vectors and its gradient by reverse mode through the normalisations.  The
 // same function and gradient are evaluated here in closed form (an identity,
@@ -87,47 +142,52 @@ __device__ __forceinline__ void project_distance(float4& pa, float4& pb, float r
 //   grad_b = -t1 grad_c - t2 grad_d,   grad_a = -(grad_b + grad_c + grad_d),
 // where t1, t2 are the projections of c and d on the hinge
 // ((c - a).e / |e|^2, (d - a).e / |e|^2).  The degeneracy gates are the
-// reference's (|e|, |A1|/|e|, |A2|/|e| above 1e-12).
-__device__ __forceinline__ void project_dihedral(float4& A, float4& B, float4& C, float4& D, float rest,
+// reference's (|e|, |A1|/|e|, |A2|/|e| above 1e-12).  False when the
+// reference skips the hinge (as project_distance).
+__device__ __forceinline__ bool project_dihedral(float4& A, float4& B, float4& C, float4& D, float rest,
                                                  float comp, float& lambda, float inv_dt2) {
-    const float3 a = f3(A), b = f3(B), c = f3(C), d = f3(D);
-    const float3 edge = b - a;
-    const float3 toC = c - a;
-    const float3 toD = d - a;
-    const float3 A1 = cross(edge, toC);
-    const float3 A2 = cross(toD, edge);
-    const float e2 = dot(edge, edge), q1 = dot(A1, A1), q2 = dot(A2, A2);
+    const float3 a = f3(A);
+    const float3 edge = rn_sub(f3(B), a);
+    const float3 toC = rn_sub(f3(C), a);
+    const float3 toD = rn_sub(f3(D), a);
+    const float3 A1 = fma_cross(edge, toC);
+    const float3 A2 = fma_cross(toD, edge);
+    const float e2 = fma_dot(edge, edge), q1 = fma_dot(A1, A1), q2 = fma_dot(A2, A2);
     const float k2 = kMinimumLengthF * kMinimumLengthF;
-    if (!(e2 > k2) || !(q1 > k2 * e2) || !(q2 > k2 * e2)) return;
-    const float iel = rsqrtf(e2);
-    const float el = e2 * iel;
-    const float sine = dot(edge, cross(A1, A2)) * iel;
-    const float cosine = dot(A1, A2);
-    const float s1 = -el * fast_rcp(q1), s2 = -el * fast_rcp(q2);
-    const float3 gc = A1 * s1;
-    const float3 gd = A2 * s2;
-    const float ie2 = iel * iel;
-    const float t1 = dot(toC, edge) * ie2, t2 = dot(toD, edge) * ie2;
-    const float3 gb = -(gc * t1 + gd * t2);
-    const float3 ga = -((gb + gc) + gd);
-    const float angle = fast_atan2(sine, cosine);
-    // The reference skips a hinge whose angle or gradient is not finite.  A
-    // non-finite gradient component makes wg (and den) non-finite, and a
-    // non-finite angle makes dl non-finite, so the two checks below reject
-    // exactly those cases without testing each component.
-    const float wg = A.w * dot(ga, ga) + B.w * dot(gb, gb) + C.w * dot(gc, gc) + D.w * dot(gd, gd);
-    const float alpha = comp * inv_dt2;
-    const float den = wg + alpha;
-    if (!(den > 0.0f) || !isfinite(den) || !isfinite(wg)) return;
-    const float value = wrap_two_pi(angle - rest);
-    const float dl = (-value - alpha * lambda) * fast_rcp(den);
-    if (!isfinite(dl)) return;
-    const float sa = A.w * dl, sb = B.w * dl, sc = C.w * dl, sd = D.w * dl;
-    A.x += sa * ga.x; A.y += sa * ga.y; A.z += sa * ga.z;
-    B.x += sb * gb.x; B.y += sb * gb.y; B.z += sb * gb.z;
-    C.x += sc * gc.x; C.y += sc * gc.y; C.z += sc * gc.z;
-    D.x += sd * gd.x; D.y += sd * gd.y; D.z += sd * gd.z;
-    lambda += dl;
+    const float gate = __fmul_rn(k2, e2);
+    bool ok = e2 > k2 && q1 > gate && q2 > gate;
+    const float iel = rsqrt_normal(e2);
+    const float el = __fmul_rn(e2, iel);
+    const float sine = __fmul_rn(fma_dot(edge, fma_cross(A1, A2)), iel);
+    const float cosine = fma_dot(A1, A2);
+    const float3 gc = rn_scale(A1, -__fmul_rn(el, rcp_normal(q1)));
+    const float3 gd = rn_scale(A2, -__fmul_rn(el, rcp_normal(q2)));
+    const float ie2 = __fmul_rn(iel, iel);
+    const float t1 = __fmul_rn(fma_dot(toC, edge), ie2), t2 = __fmul_rn(fma_dot(toD, edge), ie2);
+    const float3 gb = make_float3(-__fmaf_rn(gc.x, t1, __fmul_rn(gd.x, t2)), -__fmaf_rn(gc.y, t1, __fmul_rn(gd.y, t2)),
+                                  -__fmaf_rn(gc.z, t1, __fmul_rn(gd.z, t2)));
+    const float3 na = rn_add(rn_add(gb, gc), gd);  // -grad_a
+    const float angle = atan2_straight(sine, cosine);
+    const float wg =
+        __fmaf_rn(D.w, fma_dot(gd, gd),
+                  __fmaf_rn(C.w, fma_dot(gc, gc), __fmaf_rn(B.w, fma_dot(gb, gb), __fmul_rn(A.w, fma_dot(na, na)))));
+    const float alpha = __fmul_rn(comp, inv_dt2);
+    const float den = __fadd_rn(wg, alpha);
+    const float value = wrap_two_pi(__fadd_rn(angle, -rest));
+    const float dl = __fmul_rn(__fmaf_rn(-alpha, lambda, -value), rcp_normal(den));
+    // The reference skips a hinge whose angle or gradient is not finite: a
+    // non-finite gradient component makes den non-finite, NaN arguments of
+    // the angle show in their sum, and any other non-finite angle makes dl
+    // non-finite.
+    const float args = sine + cosine;
+    constexpr float kLargest = 3.402823466e+38f;
+    ok = ok && args == args && den > 0.0f && den <= kLargest && fabsf(dl) <= kLargest;
+    fma_add(A, -__fmul_rn(A.w, dl), na);
+    fma_add(B, __fmul_rn(B.w, dl), gb);
+    fma_add(C, __fmul_rn(C.w, dl), gc);
+    fma_add(D, __fmul_rn(D.w, dl), gd);
+    lambda = __fadd_rn(lambda, dl);
+    return ok;
 }
 
 // ---- rigid payload (suspension.cpp:538-690, 1018-1163) in FP32 -----------
@@ -496,7 +556,7 @@ __device__ __forceinline__ void run_local_stages(const DevTable& t, int kind, in
                 const uint32_t ia = v & 0xffffu, ib = v >> 16;
                 float4 pa = x[ia], pb = x[ib];
                 float lam = lambda[i];
-                project_distance(pa, pb, rest[i], comp[i], lam, inv_dt2);
+                if (!project_distance(pa, pb, rest[i], comp[i], lam, inv_dt2)) continue;
                 x[ia] = pa;
                 x[ib] = pb;
                 lambda[i] = lam;
@@ -512,7 +572,7 @@ __device__ __forceinline__ void run_local_stages(const DevTable& t, int kind, in
                 const uint32_t ia = v0 & 0xffffu, ib = v0 >> 16, ic = v1 & 0xffffu, id = v1 >> 16;
                 float4 A = x[ia], B = x[ib], C = x[ic], D = x[id];
                 float lam = lambda[i];
-                project_dihedral(A, B, C, D, rest[i], comp[i], lam, inv_dt2);
+                if (!project_dihedral(A, B, C, D, rest[i], comp[i], lam, inv_dt2)) continue;
                 x[ia] = A; x[ib] = B; x[ic] = C; x[id] = D;
                 lambda[i] = lam;
             }
@@ -529,7 +589,7 @@ __device__ __forceinline__ void run_global_colour(const DevGlobal& g, int kind, 
             const uint32_t a = __ldg(g.a + i), b = __ldg(g.b + i);
             float4 pa = __ldcg(pos + a), pb = __ldcg(pos + b);
             float lam = __ldcg(g.lambda + i);
-            project_distance(pa, pb, __ldg(g.rest + i), __ldg(g.comp + i), lam, inv_dt2);
+            if (!project_distance(pa, pb, __ldg(g.rest + i), __ldg(g.comp + i), lam, inv_dt2)) continue;
             __stcg(pos + a, pa);
             __stcg(pos + b, pb);
             __stcg(g.lambda + i, lam);
@@ -537,7 +597,7 @@ __device__ __forceinline__ void run_global_colour(const DevGlobal& g, int kind, 
             const uint32_t a = __ldg(g.a + i), b = __ldg(g.b + i), c = __ldg(g.c + i), d = __ldg(g.d + i);
             float4 A = __ldcg(pos + a), B = __ldcg(pos + b), C = __ldcg(pos + c), D = __ldcg(pos + d);
             float lam = __ldcg(g.lambda + i);
-            project_dihedral(A, B, C, D, __ldg(g.rest + i), __ldg(g.comp + i), lam, inv_dt2);
+            if (!project_dihedral(A, B, C, D, __ldg(g.rest + i), __ldg(g.comp + i), lam, inv_dt2)) continue;
             __stcg(pos + a, A); __stcg(pos + b, B); __stcg(pos + c, C); __stcg(pos + d, D);
             __stcg(g.lambda + i, lam);
         }
@@ -723,7 +783,7 @@ __global__ void __launch_bounds__(1024) xpbd_step_kernel(const __grid_constant__
                 const uint32_t a = __ldg(p.seam_a + i), c = __ldg(p.seam_b + i);
                 float4 pa = __ldcg(p.pos_out + a), pb = __ldcg(p.pos_out + c);
                 float lam = 0.0f;  // stitches are rigid: alpha = 0, lambda unused
-                project_distance(pa, pb, 0.0f, 0.0f, lam, p.inv_dt2);
+                if (!project_distance(pa, pb, 0.0f, 0.0f, lam, p.inv_dt2)) continue;
                 __stcg(p.pos_out + a, pa);
                 __stcg(p.pos_out + c, pb);
             }

@@ -44,6 +44,11 @@ cudaError_t tape_kernel_launch(const cudaLaunchConfig_t& cfg, const ClusterParam
 cudaError_t adjoint_kernel_limits(int max_dynamic_smem, bool non_portable_cluster);
 cudaError_t adjoint_kernel_launch(const cudaLaunchConfig_t& cfg, const AdjointParams& params);
 
+// Device tables of one sweep direction's hand-overs (allocations appended
+// to `owned`); the caller sets the shared-memory offsets.
+ClusterFlowDev upload_flow(const ClusterSchedule& s, const ClusterFlow& f, std::vector<void*>& owned,
+                           cudaStream_t stream);
+
 // Status words written by the step kernels -> status and message.
 swb_status decode_status(const int status[2], std::string& message);
 
@@ -77,6 +82,7 @@ struct StructureImpl {
     LineContactDev lines_host{};
     LineContactDev* d_lines = nullptr;
     int threads = 0;
+    int reverse_threads = 0;  // of a rollout's reverse step
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::vector<void*> owned;
