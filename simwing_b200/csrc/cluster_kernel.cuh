@@ -495,6 +495,8 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_kernel_t(const __gri
         cctx.grid = p.grid;
         cctx.grid.status = I.status;
         cctx.grid.blocks = gridDim.x;
+        cctx.order = smem_addr(smem + I.smem_order);
+        cctx.order_bytes = I.order_bytes;
         // multipliers and records restart every substep (beginContactSubstep,
         // contact.cpp:1043-1055)
         if (me == 0 && tid == 0) {

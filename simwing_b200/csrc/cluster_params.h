@@ -46,8 +46,7 @@ struct ContactQuery {
     double normal[3];        // closest-feature normal (not yet oriented)
     double ccd_normal[3];    // normal of the swept query's geometry
     double eff;              // effective inverse mass sum w_i m_i^-1 w_i
-    uint32_t addr[6];        // cluster shared-memory addresses of the nodes: first, then second primitive
-    uint32_t slot[6];        // their slots
+    uint32_t slot[6];        // slots of the nodes: first, then second primitive
     float inv[6];            // their inverse masses
     uint32_t ccd_state;      // SWB_CCD_*
     uint32_t certified;      // the snapshot geometry is certified
@@ -73,7 +72,7 @@ struct ContactRecordDev {
     double normal[3];
     double lambda;
     double eff;              // effective inverse mass
-    uint32_t addr[6];        // node addresses and slots, as in ContactQuery
+    uint32_t addr[6];        // cluster shared-memory addresses of the nodes: first, then second primitive
     uint32_t slot[6];
     float inv[6];
     uint32_t fc, sc;
@@ -228,6 +227,7 @@ struct ClusterInstance {
     const uint32_t* pair_rec;
     // Fabric self-contact, or nullptr.  Single-structure launches only.
     const ContactDev* contact;
+    uint32_t smem_order, order_bytes;  // shared memory of the key-ordered passes (byte offset and size)
     // Line-line contact (swb_structure_set_line_contact), or nullptr.
     // Single-structure launches only.
     const LineContactDev* lines;

@@ -95,6 +95,8 @@ struct ContactCtx {
     uint32_t grank, gctas;
     int helpers;
     GridBarrier grid;
+    uint32_t order;            // shared memory of the key-ordered passes (run_order): address
+    uint32_t order_bytes;
 };
 
 // The barrier between two detection phases.
@@ -628,42 +630,174 @@ __device__ __noinline__ void cluster_order(const ContactCtx& c, cooperative_grou
     cluster.sync();
 }
 
-// Runs work(id[item]) (work(item) without `id`) for `items` items in an
-// order that keeps, for every node, the items touching it in item order
-// (the calling block, after cluster_order): rounds, each running together
-// the items whose earlier neighbours have all run (they share no node), a
-// block barrier after each.  The nodes may live in any CTA of the cluster,
-// but only this block's threads touch them until the cluster barrier that
-// follows, so the block barrier orders one round's writes before the next
-// round's reads.  Every item ends a round with all its links released, so a
-// round runs at least one item and there are at most `items` rounds.
-template <class Work>
-__device__ __forceinline__ void run_order(const ContactDev& C, uint32_t items, const uint32_t* id, Work work) {
-    __shared__ uint32_t front_n[2];
-    uint32_t* front[2] = {C.lv_front, C.lv_front + C.cand_cap};
-    if (threadIdx.x < 2) front_n[threadIdx.x] = 0;
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < items; i += blockDim.x)
-        if (__ldcg(C.lv_npred + i) == 0u) front[0][atomicAdd(&front_n[0], 1u)] = i;
-    __syncthreads();
-    uint32_t done = 0;
-    for (uint32_t r = 0; r < items && done < items; ++r) {
-        const uint32_t cur = r & 1u, n = front_n[cur];
-        for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) {
-            const uint32_t i = front[cur][k];
-            work(id ? id[i] : i);
-            const uint32_t m = C.lv_nsucc[i];
-            for (uint32_t q = 0; q < m; ++q) {
-                const uint32_t j = C.lv_succ[static_cast<size_t>(i) * 6 + q];
-                if (atomicSub(&C.lv_npred[j], 1u) == 1u) front[cur ^ 1u][atomicAdd(&front_n[cur ^ 1u], 1u)] = j;
-            }
-        }
-        done += n;
-        __syncthreads();
-        if (threadIdx.x == 0) front_n[cur] = 0;
-        // read by every thread before the reset above takes effect two
-        // rounds later: the next round's barrier separates them
+// A key-ordered pass works on an item with a group of lanes: four nodes by
+// three components (a feature has four nodes: a vertex and a triangle, or two
+// edges), the fourth lane of each node idle.
+constexpr uint32_t kGroup = 16;
+struct GroupLane {
+    uint32_t mask;   // the group's lanes of the warp
+    uint32_t lane;   // 0..15
+    uint32_t node, comp;
+};
+__device__ __forceinline__ GroupLane group_lane() {
+    GroupLane g;
+    g.lane = threadIdx.x & (kGroup - 1);
+    g.mask = 0xffffu << (threadIdx.x & 16u);
+    g.node = g.lane >> 2;
+    g.comp = g.lane & 3u;
+    return g;
+}
+
+// The weighted points of a feature's two primitives, component g.comp: the
+// first of the group's four nodes the first primitive's (fc of them), summed
+// node after node; `p`: the lane's node's component, w: the four weights.
+__device__ __forceinline__ void group_points(const GroupLane& g, double p, const double w[4], uint32_t fc, double& first,
+                                             double& second) {
+    const double a = __shfl_sync(g.mask, p, g.comp, kGroup), b = __shfl_sync(g.mask, p, 4 + g.comp, kGroup),
+                 c = __shfl_sync(g.mask, p, 8 + g.comp, kGroup), d = __shfl_sync(g.mask, p, 12 + g.comp, kGroup);
+    if (fc == 1) {
+        first = w[0] * a;
+        second = w[3] * d + (w[2] * c + w[1] * b);
+    } else {
+        first = w[1] * b + w[0] * a;
+        second = w[3] * d + w[2] * c;
     }
+}
+__device__ __forceinline__ D3 group_vector(const GroupLane& g, double v) {
+    return {__shfl_sync(g.mask, v, 0, kGroup), __shfl_sync(g.mask, v, 1, kGroup), __shfl_sync(g.mask, v, 2, kGroup)};
+}
+__device__ __forceinline__ float ld_component(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_component(uint32_t addr, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+// Brings the 128-byte line at `p` into the L1 cache: four asynchronous copies
+// of four bytes, one per sector, to a place in shared memory nobody reads
+// (a prefetch instruction left the reads at L2's latency).
+__device__ __forceinline__ void fetch_line(uint32_t sink, const void* p) {
+    const char* q = static_cast<const char*>(p);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sink + 4u * k), "l"(q + 32 * k));
+}
+__device__ __forceinline__ uint32_t lds_u16(uint32_t addr) {
+    uint16_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sts_u16(uint32_t addr, uint32_t v) {
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"(static_cast<uint16_t>(v)) : "memory");
+}
+__device__ __forceinline__ uint32_t atom_shared_add(uint32_t addr, uint32_t v) {
+    uint32_t old;
+    asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(addr), "r"(v) : "memory");
+    return old;
+}
+
+// The links of run_order in shared memory: per item its followers (0xffff:
+// none), the count of items it still waits for, a place in the queue.
+constexpr uint32_t kOrderItemBytes = 11;
+constexpr uint32_t kOrderSink = 32;  // bytes before them: where fetch_line's copies go
+// Runs work(item) for `items` items in an order that keeps, for every node,
+// the items touching it in item order (the calling block, after
+// cluster_order): rounds, each running together the items whose earlier
+// neighbours have all run (they share no node), a barrier after each.  The
+// nodes may live in any CTA of the cluster, but only this block's threads
+// touch them until the cluster barrier that follows, so the block's barrier
+// orders one round's writes before the next round's reads.  Every item ends
+// a round with all its links released, so a round runs at least one item and
+// there are at most `items` rounds.  A group of lanes runs an item;
+// ahead(item), on one lane, brings the data of an item whose turn is near
+// closer.
+//
+// A round is a chain of dependent accesses and FP64 arithmetic, which is why
+// the links are copied to shared memory when they fit (a link released there
+// costs tens of cycles, an atomic in L2 several hundred; larger passes keep
+// them in global memory), an item's data lies in one cache line fetched two
+// rounds ahead, and the lanes of a group share its arithmetic.  A landed 24 x
+// 24 sheet has 3,900 candidates in contact in 270 rounds; per round: links
+// and data read from L2 in turn, one thread an item, 7.3 us; links in shared
+// memory and one line per item 3.0 us; groups of lanes, the first lines
+// fetched ahead, 2.4 us with 256 threads and 2.0 us with the whole block
+// (wide rounds in fewer turns).
+template <class Work, class Ahead>
+__device__ __forceinline__ void run_order(const ContactCtx& c, uint32_t items, Work work, Ahead ahead) {
+    const ContactDev& C = *c.C;
+    __shared__ uint32_t round_n[3];  // items of this round, of the next one, the count being cleared
+    const bool shared = items < 0xffffu && kOrderSink + (items + 8) * kOrderItemBytes <= c.order_bytes;
+    const uint32_t sink = c.order;
+    const uint32_t succ = c.order + kOrderSink, near_queue = succ + 8 * items,
+                   near_waits = (near_queue + 2 * items + 3) & ~3u;  // a byte per item
+    if (threadIdx.x < 3) round_n[threadIdx.x] = 0;
+    if (shared)
+        for (uint32_t i = threadIdx.x; i < (items + 3) / 4; i += blockDim.x)
+            asm volatile("st.shared.u32 [%0], %1;" ::"r"(near_waits + 4 * i), "r"(0u) : "memory");
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < items; i += blockDim.x) {
+        const uint32_t waits = __ldcg(C.lv_npred + i);
+        if (shared) {
+            const uint32_t m = __ldcg(C.lv_nsucc + i);
+            if (waits) atom_shared_add(near_waits + (i & ~3u), waits << (8 * (i & 3u)));
+            for (uint32_t q = 0; q < 4; ++q)
+                sts_u16(succ + 8 * i + 2 * q, q < m ? __ldcg(C.lv_succ + static_cast<size_t>(i) * 6 + q) : 0xffffu);
+        }
+        if (waits == 0u) {
+            const uint32_t at = atomicAdd(&round_n[0], 1u);
+            if (shared)
+                sts_u16(near_queue + 2 * at, i);
+            else
+                C.lv_front[at] = i;
+            ahead(i, sink);
+        }
+    }
+    __syncthreads();
+    const uint32_t groups = blockDim.x / kGroup;
+    {
+        const GroupLane g = group_lane();
+        const uint32_t group = threadIdx.x / kGroup;
+        constexpr uint32_t kNone = ~0u;
+        // follower q of item i
+        auto follower = [&](uint32_t i, uint32_t q) -> uint32_t {
+            if (shared) {
+                const uint32_t j = lds_u16(succ + 8 * i + 2 * q);
+                return j == 0xffffu ? kNone : j;
+            }
+            return q < C.lv_nsucc[i] ? C.lv_succ[static_cast<size_t>(i) * 6 + q] : kNone;
+        };
+        // one wait of item j less; true when it was the last
+        auto release = [&](uint32_t j) {
+            if (!shared) return atomicSub(&C.lv_npred[j], 1u) == 1u;
+            const uint32_t shift = 8 * (j & 3u);
+            return ((atom_shared_add(near_waits + (j & ~3u), 0u - (1u << shift)) >> shift) & 0xffu) == 1u;
+        };
+        uint32_t done = 0;  // the queue's items before this round
+        for (uint32_t r = 0; r < items && done < items; ++r) {
+            const uint32_t n = round_n[r % 3];
+            uint32_t* next_n = &round_n[(r + 1) % 3];
+            if (threadIdx.x == 0) round_n[(r + 2) % 3] = 0;
+            for (uint32_t k = group; k < n; k += groups) {
+                const uint32_t i = shared ? lds_u16(near_queue + 2 * (done + k)) : C.lv_front[done + k];
+                // lane 4 q + t: follower q, and its follower t
+                const uint32_t j = follower(i, g.node);
+                const uint32_t jj = j != kNone ? follower(j, g.comp) : kNone;
+                if (jj != kNone) ahead(jj, sink);
+                work(i, g);
+                if (g.comp == 0 && j != kNone && release(j)) {
+                    const uint32_t at = done + n + atomicAdd(next_n, 1u);
+                    if (shared)
+                        sts_u16(near_queue + 2 * at, j);
+                    else
+                        C.lv_front[at] = j;
+                }
+            }
+            done += n;
+            __syncthreads();
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 }
 
@@ -678,90 +812,133 @@ __device__ __forceinline__ uint32_t carried_flags(uint32_t f) {
     return ((f & kEntryRecord) && (f & kEntryApplied)) ? (kEntryRecord | kEntryApplied) : 0u;
 }
 
-// One candidate's projection (contact.cpp:1318-1457): warm start from its
-// entry of the previous table (copied into cand_entry beforehand), the XPBD
-// normal projection on the live nodes, its entry for the next table.
-static __device__ __noinline__ void project_one(const ContactCtx& c, uint32_t i) {
+// One candidate in contact as its projection wants it: one cache line, in
+// hit order (kept in the certification's scratch, which is idle during the
+// iterations).  The first `fc` nodes are the first primitive's; fc = 0 when
+// the candidate has failed.
+struct __align__(128) ContactWork {
+    double2 w[2];       // the nodes' closest-feature weights
+    double2 normal_xy;  // oriented
+    double2 normal_z_eff;
+    uint32_t addr[4];
+    float inv[4];
+    double lambda;      // the warm start
+    uint32_t fc_flags;  // fc | the warm start entry's flags << 8
+    uint32_t cand;      // candidate index
+    double2 pad;
+};
+static_assert(sizeof(ContactWork) == 128 && sizeof(ContactWork) <= sizeof(ContactRecordDev));
+
+__device__ __forceinline__ ContactWork* contact_work(const ContactDev& C) {
+    return reinterpret_cast<ContactWork*>(C.cand_rec);
+}
+
+// The work record of hit `h` (candidate i): the checks and the orientation
+// the projection starts with (contact.cpp:1318-1351), and its nodes'
+// addresses.
+static __device__ __noinline__ void prepare_work(const ContactCtx& c, uint32_t h, uint32_t i) {
     const ContactDev& C = *c.C;
-    const ContactQuery& Q = C.query[i];
-    ContactEntry& out = C.cand_entry[i];
-    ContactEntry e = out;  // the warm start
+    ContactQuery& Q = C.query[i];
+    const ContactEntry& e = C.cand_entry[i];
+    uint32_t live = 0;
+    D3 normal = d3_of(Q.normal);
     if (!Q.certified) {
         contact_fail_at(C, c.status, kContactGeometry, C.cand[i]);
-        return;
+    } else {
+        if (contact::dot(normal, d3_of(Q.ccd_normal)) < 0.0) normal = -normal;
+        if (!contact::finite3(normal) || fabs(contact::norm2(normal) - 1.0) > 1.0e-8)
+            contact_fail_at(C, c.status, kContactNormal, C.cand[i]);
+        else
+            live = Q.fc;
     }
-    D3 normal = d3_of(Q.normal);
-    if (contact::dot(normal, d3_of(Q.ccd_normal)) < 0.0) normal = -normal;
-    if (!contact::finite3(normal) || fabs(contact::norm2(normal) - 1.0) > 1.0e-8) {
-        contact_fail_at(C, c.status, kContactNormal, C.cand[i]);
-        return;
-    }
-    const double dt = c.dt;
-    const double alpha = C.compliance / (dt * dt);
-    const double margin = contact::dmax(0.1 * C.separation, 8.0 * C.ccd.distance_tolerance);
-    const uint32_t fc = Q.fc, sc = Q.sc;
-    // the first primitive's nodes in A, the second's in B (constant indices)
-    float4 A[3], B[3];
+    const int fc = static_cast<int>(Q.fc);
+    ContactWork W;
+    double w[4];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        if (k < static_cast<int>(fc)) A[k] = ld_node(Q.addr[k]);
-        if (k < static_cast<int>(sc)) B[k] = ld_node(Q.addr[fc + k]);
+    for (int k = 0; k < 4; ++k) {
+        W.addr[k] = slot_addr(c, Q.slot[k]);
+        W.inv[k] = Q.inv[k];
+        w[k] = fc == 1 ? (k == 0 ? Q.fw[0] : Q.sw[k > 0 ? k - 1 : 0]) : (k < 2 ? Q.fw[k] : Q.sw[k - 2]);
     }
-    auto point = [&](const float4* P, uint32_t count, const double* w) {
-        D3 r{0.0, 0.0, 0.0};
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            if (k < static_cast<int>(count)) r = r + w[k] * world_of(c, P[k]);
-        return r;
-    };
-    const double gap = contact::dot(point(A, fc, Q.fw) - point(B, sc, Q.sw), normal) - C.separation;
-    const double eff = Q.eff;
-    if ((gap > margin && e.lambda == 0.0) || !(eff + alpha > 0.0)) {
-        if (!(eff + alpha > 0.0) && gap < 0.0 && !(gap > margin && e.lambda == 0.0)) {
-            contact_fail_at(C, c.status, kContactNoResponse, C.cand[i]);
-            return;
+    W.w[0] = make_double2(w[0], w[1]);
+    W.w[1] = make_double2(w[2], w[3]);
+    W.normal_xy = make_double2(normal.x, normal.y);
+    W.normal_z_eff = make_double2(normal.z, Q.eff);
+    W.lambda = e.lambda;
+    W.fc_flags = live | e.flags << 8;
+    W.cand = i;
+    W.pad = make_double2(0.0, 0.0);
+    contact_work(C)[h] = W;
+}
+
+// One candidate's projection (contact.cpp:1352-1457) by a group of lanes: warm
+// start from its entry of the previous table (copied into cand_entry
+// beforehand), the XPBD normal projection on the live nodes, its entry for
+// the next table.
+// What a projection needs beside its work record, held in registers.
+struct ProjectConst {
+    double alpha, margin, separation, dt;
+    double origin;        // of the lane's component
+    const ContactDev* C;
+    ContactEntry* entry;  // by candidate
+    int* status;
+};
+__device__ __forceinline__ void project_one(const ContactWork& W, const ProjectConst& pc, const GroupLane& g) {
+    const uint32_t home = W.addr[g.node];
+    const double2 w01 = W.w[0], w23 = W.w[1], nxy = W.normal_xy, nze = W.normal_z_eff;
+    const double lambda = W.lambda;
+    const uint32_t ff = W.fc_flags, cand = W.cand;
+    const float inv = W.inv[g.node];
+    const uint32_t fc = ff & 0xffu, flags = ff >> 8;
+    if (fc == 0) return;
+    const uint32_t addr = home + 4u * g.comp;
+    const float x = ld_component(addr);
+    const double w[4] = {w01.x, w01.y, w23.x, w23.y};
+    const double eff = nze.y, alpha = pc.alpha;
+    const D3 normal{nxy.x, nxy.y, nze.x};
+    const double world = pc.origin + static_cast<double>(x);
+    double first, second;
+    group_points(g, world, w, fc, first, second);
+    const double gap = contact::dot(group_vector(g, first - second), normal) - pc.separation;
+    ContactEntry& out = pc.entry[cand];
+    if ((gap > pc.margin && lambda == 0.0) || !(eff + alpha > 0.0)) {
+        if (g.lane == 0) {
+            if (!(eff + alpha > 0.0) && gap < 0.0 && !(gap > pc.margin && lambda == 0.0))
+                contact_fail_at(*pc.C, pc.status, kContactNoResponse, pc.C->cand[cand]);
+            else
+                out.flags = carried_flags(flags);
         }
-        e.flags = carried_flags(e.flags);
-        out = e;
         return;
     }
-    const double delta = (-gap - alpha * e.lambda) / (eff + alpha);
-    const double next = contact::dmax(0.0, e.lambda + delta);
-    const double applied = next - e.lambda;
+    const double delta = (-gap - alpha * lambda) / (eff + alpha);
+    const double next = contact::dmax(0.0, lambda + delta);
+    const double applied = next - lambda;
     if (!isfinite(next) || !isfinite(applied)) {
-        contact_fail_at(C, c.status, kContactProjection, C.cand[i]);
+        if (g.lane == 0) contact_fail_at(*pc.C, pc.status, kContactProjection, pc.C->cand[cand]);
         return;
     }
     // impulse w (applied / dt) n on the first primitive, the opposite on the
     // second; positions move by m^-1 dt impulse (contact.cpp:1404-1417)
-    auto move = [&](float4& X, double w, float inv, uint32_t addr) {
-        const D3 impulse = (w * (applied / dt)) * normal;
-        const D3 p = world_of(c, X) + impulse * (static_cast<double>(inv) * dt);
-        X.x = static_cast<float>(p.x - c.o[0]);
-        X.y = static_cast<float>(p.y - c.o[1]);
-        X.z = static_cast<float>(p.z - c.o[2]);
-        st_node(addr, X);
-    };
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-        if (k < static_cast<int>(fc)) move(A[k], Q.fw[k], Q.inv[k], Q.addr[k]);
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-        if (k < static_cast<int>(sc)) move(B[k], -Q.sw[k], Q.inv[fc + k], Q.addr[fc + k]);
-    const D3 fp = point(A, fc, Q.fw), sp = point(B, sc, Q.sw);
-    const double solved = contact::dot(fp - sp, normal) - C.separation;
-    if (!contact::finite3(fp) || !contact::finite3(sp) || !isfinite(solved)) {
-        contact_fail_at(C, c.status, kContactSolved, C.cand[i]);
+    const double rate = applied / pc.dt;
+    const double own = g.node == 0 ? w[0] : (g.node == 1 ? w[1] : (g.node == 2 ? w[2] : w[3]));
+    const double weight = g.node < fc ? own : -own;
+    const double along = g.comp == 0 ? normal.x : (g.comp == 1 ? normal.y : normal.z);
+    const double impulse = (weight * rate) * along;
+    const double moved = world + impulse * (static_cast<double>(inv) * pc.dt);
+    const float to = static_cast<float>(moved - pc.origin);
+    if (g.comp < 3) st_component(addr, to);
+    // the solved points and gap are finite when the moved nodes are
+    if (__any_sync(g.mask, g.comp < 3 && !isfinite(to))) {
+        if (g.lane == 0) contact_fail_at(*pc.C, pc.status, kContactSolved, pc.C->cand[cand]);
         return;
     }
     // a record continuing from the previous iteration keeps its impulse
     // ledger; a new one starts it (contact.cpp:1391-1401); visited, it is a
     // record of this iteration
-    const bool ledger = (e.flags & kEntryRecord) && (e.flags & kEntryApplied);
-    e.lambda = next;
-    e.flags = kEntryRecord | ((ledger || applied != 0.0) ? kEntryApplied : 0u);
-    e.normal[0] = normal.x; e.normal[1] = normal.y; e.normal[2] = normal.z;
-    out = e;
+    const bool ledger = (flags & kEntryRecord) && (flags & kEntryApplied);
+    if (g.node == 0 && g.comp < 3) out.normal[g.comp] = along;
+    if (g.lane == 3) out.lambda = next;
+    if (g.lane == 4) out.flags = kEntryRecord | ((ledger || applied != 0.0) ? kEntryApplied : 0u);
 }
 
 // The contact iteration's projections in key order (rounds of candidates
@@ -816,12 +993,9 @@ __device__ __noinline__ void contact_project(const ContactCtx& c, cooperative_gr
     cluster.sync();
     if (!contact_failed(c.status)) {  // uniform: read after the barrier
         const uint32_t hits = C.mark_a[count];
-        // cluster addresses of the nodes of the candidates in contact (read
-        // by rank 0's rounds after cluster_order's barriers)
-        for (uint32_t h = gt; h < hits; h += stride) {
-            ContactQuery& Q = C.query[C.hit[h]];
-            for (uint32_t j = 0; j < Q.fc + Q.sc; ++j) Q.addr[j] = slot_addr(c, Q.slot[j]);
-        }
+        // the work records of the candidates in contact (read by rank 0's
+        // rounds after cluster_order's barriers)
+        for (uint32_t h = gt; h < hits; h += stride) prepare_work(c, h, C.hit[h]);
         cluster_order(c, cluster, hits, slots, [&](uint32_t h, uint32_t* s) -> uint32_t {
             const ContactQuery& Q = C.query[C.hit[h]];
             const uint32_t n = Q.fc + Q.sc;
@@ -829,7 +1003,21 @@ __device__ __noinline__ void contact_project(const ContactCtx& c, cooperative_gr
             for (int j = 0; j < 6; ++j) s[j] = j < static_cast<int>(n) ? Q.slot[j] : 0u;
             return n;
         });
-        if (c.me == 0) run_order(C, hits, C.hit, [&](uint32_t i) { project_one(c, i); });
+        if (c.me == 0) {
+            const ContactWork* work = contact_work(C);
+            const uint32_t comp = threadIdx.x & 3u;
+            const ProjectConst pc{C.compliance / (c.dt * c.dt),
+                                  contact::dmax(0.1 * C.separation, 8.0 * C.ccd.distance_tolerance),
+                                  C.separation,
+                                  c.dt,
+                                  comp == 0 ? c.o[0] : (comp == 1 ? c.o[1] : c.o[2]),
+                                  &C,
+                                  C.cand_entry,
+                                  c.status};
+            run_order(
+                c, hits, [&](uint32_t h, const GroupLane& g) { project_one(work[h], pc, g); },
+                [&](uint32_t h, uint32_t sink) { fetch_line(sink, work + h); });
+        }
     }
     cluster.sync();
     if (contact_failed(c.status)) return;  // uniform: read after the barrier
@@ -891,7 +1079,11 @@ __device__ __noinline__ void contact_certify_all(const ContactCtx& c, cooperativ
         D3 normal = d3_of(Q.normal);
         if (contact::dot(normal, impact ? d3_of(Q.ccd_normal) : d3_of(e->normal)) < 0.0) normal = -normal;
         const uint32_t fc = Q.fc, sc = Q.sc;
-        const D3 fp = weighted_live(c, Q.addr, fc, Q.fw), sp = weighted_live(c, Q.addr + fc, sc, Q.sw);
+        uint32_t addr[6];
+#pragma unroll
+        for (int j = 0; j < 6; ++j) addr[j] = j < static_cast<int>(fc + sc) ? slot_addr(c, Q.slot[j]) : 0u;
+        const uint32_t* second = fc == 1 ? addr + 1 : addr + 2;
+        const D3 fp = weighted_live(c, addr, fc, Q.fw), sp = weighted_live(c, second, sc, Q.sw);
         const double gap = contact::dot(fp - sp, normal) - C.separation;
         if (impact && (!contact::finite3(fp) || !contact::finite3(sp) || !contact::finite3(normal) || !isfinite(gap))) {
             contact_fail_at(C, c.status, kContactFinalNonFinite, code);
@@ -909,7 +1101,7 @@ __device__ __noinline__ void contact_certify_all(const ContactCtx& c, cooperativ
             r.sw[j] = Q.sw[j];
         }
         for (int j = 0; j < 6; ++j) {
-            r.addr[j] = j < static_cast<int>(fc + sc) ? slot_addr(c, Q.slot[j]) : 0u;
+            r.addr[j] = addr[j];
             r.slot[j] = Q.slot[j];
             r.inv[j] = Q.inv[j];
         }
@@ -946,43 +1138,30 @@ __device__ __noinline__ void contact_certify_all(const ContactCtx& c, cooperativ
 }
 
 // Coulomb friction of one certified record on the finalized velocities
-// (contact.cpp:2081-2147).
-static __device__ __noinline__ void friction_one(const ContactCtx& c, const ContactRecordDev& r) {
+// (contact.cpp:2081-2147) by a group of lanes.
+static __device__ __noinline__ void friction_one(const ContactCtx& c, const ContactRecordDev& r, const GroupLane& g) {
     const ContactDev& C = *c.C;
-    const uint32_t fc = r.fc, sc = r.sc;
-    float4 A[3], B[3];
+    const uint32_t fc = r.fc;
+    const uint32_t addr = r.addr[g.node] + c.v_delta + 4u * g.comp;
+    const float v = ld_component(addr);
+    double w[4];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        if (k < static_cast<int>(fc)) A[k] = ld_node(r.addr[k] + c.v_delta);
-        if (k < static_cast<int>(sc)) B[k] = ld_node(r.addr[fc + k] + c.v_delta);
-    }
-    D3 vf{0.0, 0.0, 0.0}, vs{0.0, 0.0, 0.0};
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        if (k < static_cast<int>(fc)) vf = vf + r.fw[k] * D3{A[k].x, A[k].y, A[k].z};
-        if (k < static_cast<int>(sc)) vs = vs + r.sw[k] * D3{B[k].x, B[k].y, B[k].z};
-    }
-    const contact::Friction fr = contact::coulomb_friction(vf - vs, d3_of(r.normal), r.eff, r.lambda / c.dt,
-                                                           C.static_mu, C.dynamic_mu, r.active != 0);
+    for (int k = 0; k < 4; ++k)
+        w[k] = fc == 1 ? (k == 0 ? r.fw[0] : r.sw[k > 0 ? k - 1 : 0]) : (k < 2 ? r.fw[k] : r.sw[k - 2]);
+    double first, second;
+    group_points(g, static_cast<double>(v), w, fc, first, second);
+    const contact::Friction fr = contact::coulomb_friction(group_vector(g, first - second), d3_of(r.normal), r.eff,
+                                                           r.lambda / c.dt, C.static_mu, C.dynamic_mu, r.active != 0);
     if (!contact::finite3(fr.impulse) || !isfinite(fr.work) ||
         fr.work > 1.0e-12 * contact::dmax(1.0, contact::norm2(fr.initial_tangent))) {
-        contact_fail_at(C, c.status, kContactFriction, r.code);
+        if (g.lane == 0) contact_fail_at(C, c.status, kContactFriction, r.code);
         return;
     }
     if (fr.state == contact::kFrictionInactive) return;  // no impulse
-    auto kick = [&](float4& V, double w, float inv, uint32_t addr) {
-        const D3 dv = (w * fr.impulse) * static_cast<double>(inv);
-        V.x = static_cast<float>(V.x + dv.x);
-        V.y = static_cast<float>(V.y + dv.y);
-        V.z = static_cast<float>(V.z + dv.z);
-        st_node(addr + c.v_delta, V);
-    };
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-        if (k < static_cast<int>(fc)) kick(A[k], r.fw[k], r.inv[k], r.addr[k]);
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-        if (k < static_cast<int>(sc)) kick(B[k], -r.sw[k], r.inv[fc + k], r.addr[fc + k]);
+    const double weight = g.node < fc ? w[g.node] : -w[g.node];
+    const double along = g.comp == 0 ? fr.impulse.x : (g.comp == 1 ? fr.impulse.y : fr.impulse.z);
+    const double dv = (weight * along) * static_cast<double>(r.inv[g.node]);
+    if (g.comp < 3) st_component(addr, static_cast<float>(v + dv));
 }
 
 // ---- the three contact steps of a substep ------------------------------------
@@ -1056,7 +1235,14 @@ __device__ __forceinline__ void contact_friction(const ContactCtx& c, cooperativ
         for (int j = 0; j < 6; ++j) s[j] = j < static_cast<int>(n) ? r.slot[j] : 0u;
         return n;
     });
-    if (c.me == 0) run_order(C, records, nullptr, [&](uint32_t i) { friction_one(c, C.records[i]); });
+    if (c.me == 0)
+        run_order(
+            c, records, [&](uint32_t i, const GroupLane& g) { friction_one(c, C.records[i], g); },
+            [&](uint32_t i, uint32_t sink) {
+                const char* r = reinterpret_cast<const char*>(C.records + i);
+                fetch_line(sink, r);
+                fetch_line(sink, r + sizeof(ContactRecordDev) - 128);
+            });
     cluster.sync();
 }
 

@@ -657,6 +657,19 @@ void StructureImpl::upload_cluster_tables() {
     base.flow.smem_barriers = layout.barriers;
     base.flow.smem_bytes = layout.bytes;
     cluster_smem = layout.total;
+    if (def.has_contact) {
+        // the links of the key-ordered contact passes, beside the patch
+        base.smem_order = layout.total;
+        const size_t rows = contact_surface.vertices.size() + contact_surface.edges.size();
+        const size_t want = layout.total + rows * kContactLinkBytes + 256;
+        size_t limit = kContactSharedSteps[0];
+        for (size_t step : kContactSharedSteps)
+            if (limit < want && step >= want) limit = step;
+        limit = std::min(limit, smem_cap);
+        base.order_bytes =
+            static_cast<uint32_t>(std::max<size_t>(limit > layout.total ? (limit - layout.total) & ~size_t{15} : 0, 32));
+        cluster_smem += base.order_bytes;
+    }
     base.seam_offsets = dupload(owned, csched.seam_offsets, stream);
     base.seam_ab = dupload(owned, csched.seam_ab, stream);
     base.seam_stages = csched.seam_stages;
