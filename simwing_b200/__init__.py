@@ -697,7 +697,7 @@ class Structure:
 
     def node_states(self) -> np.ndarray:
         """(n, 3, 3) array: position, previous position, velocity."""
-        out = np.zeros((self.node_count, 3, 3), dtype=np.float64)
+        out = np.empty((self.node_count, 3, 3), dtype=np.float64)
         _check(self._lib.swb_structure_read_nodes(self._h, out.ctypes.data, self.node_count))
         return out
 

@@ -285,6 +285,7 @@ swb_status swb_structure_restore(swb_structure* s, const void* buffer, uint64_t 
         }
         cuda_check(cudaStreamSynchronize(m.stream), "restore");
         m.pending = pending;
+        m.pending_any = true;
         m.forces_dirty = true;
         m.last_applied = last;
         if (pressure != m.pressure) {

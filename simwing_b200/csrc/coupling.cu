@@ -114,9 +114,10 @@ swb_status advance(swb_coupling* c, const double* a, const double* b, double sca
         cuda_check(cudaSetDevice(S.device), "cudaSetDevice");
         const uint32_t slots = static_cast<uint32_t>(S.def.nodes.size());
         // the loads pending before the call, by slot (cleared when none is)
-        const bool any_pending = std::any_of(S.pending.begin(), S.pending.end(), [](const swb_vec3& f) {
-            return f.x != 0.0 || f.y != 0.0 || f.z != 0.0;
-        });
+        const bool any_pending = S.pending_any &&
+                                 std::any_of(S.pending.begin(), S.pending.end(), [](const swb_vec3& f) {
+                                     return f.x != 0.0 || f.y != 0.0 || f.z != 0.0;
+                                 });
         if (any_pending) {
             c->pending_host.assign(3 * static_cast<size_t>(slots), 0.0);
             for (uint64_t n = 0; n < S.def.nodes.size(); ++n) {
@@ -137,13 +138,19 @@ swb_status advance(swb_coupling* c, const double* a, const double* b, double sca
                                                                         c->d_pending, a, b, scale, endpoints,
                                                                         S.d_force, total64, c->d_flag);
         cuda_check(cudaGetLastError(), "gather_loads_kernel");
-        int flag = 0;
-        cuda_check(cudaMemcpyAsync(&flag, c->d_flag, sizeof(int), cudaMemcpyDeviceToHost, S.stream), "read");
+        cuda_check(cudaMemcpyAsync(&S.h_reads->flag, c->d_flag, sizeof(int), cudaMemcpyDeviceToHost, S.stream), "read");
         cuda_check(cudaStreamSynchronize(S.stream), "gather");
-        if (flag) {
+        if (S.h_reads->flag) {
             S.forces_dirty = true;  // the device buffer no longer holds the pending loads
             raise(SWB_INVALID_ARGUMENT, "time-integrated transfer has invalid nodal bindings or non-finite loads");
         }
+        // the applied total, in node order, read back with the step's results
+        static_assert(sizeof(swb_vec3) == 3 * sizeof(double), "swb_vec3 layout");
+        applied_total_kernel<<<1, 1024, 0, S.stream>>>(S.def.nodes.size(), c->d_items + c->bindings, total64,
+                                                       c->d_applied);
+        cuda_check(cudaGetLastError(), "applied_total_kernel");
+        cuda_check(cudaMemcpyAsync(S.h_reads->applied, c->d_applied, sizeof(S.h_reads->applied), cudaMemcpyDeviceToHost,
+                                   S.stream), "read");
         S.device_forces = true;
         try {
             S.step(*settings, 1, out);
@@ -153,15 +160,7 @@ swb_status advance(swb_coupling* c, const double* a, const double* b, double sca
             throw;
         }
         S.device_forces = false;
-        // the step consumed the loads: the applied total, in node order
-        static_assert(sizeof(swb_vec3) == 3 * sizeof(double), "swb_vec3 layout");
-        applied_total_kernel<<<1, 1024, 0, S.stream>>>(S.def.nodes.size(), c->d_items + c->bindings, total64,
-                                                       c->d_applied);
-        cuda_check(cudaGetLastError(), "applied_total_kernel");
-        swb_vec3 applied{};
-        cuda_check(cudaMemcpyAsync(&applied, c->d_applied, sizeof(applied), cudaMemcpyDeviceToHost, S.stream),
-                   "read");
-        cuda_check(cudaStreamSynchronize(S.stream), "applied");
+        const swb_vec3 applied{S.h_reads->applied[0], S.h_reads->applied[1], S.h_reads->applied[2]};
         S.last_applied = applied;
         S.forces_dirty = true;  // the buffer holds this call's loads; pending is empty again
         if (out) out->last_applied_external_force = applied;

@@ -9,6 +9,7 @@
 #include "step_params.h"
 
 #include <string>
+#include <mutex>
 #include <vector>
 
 namespace swb {
@@ -69,6 +70,22 @@ constexpr uint32_t kContactHelperRows = 16384;
 constexpr size_t kContactSharedSteps[] = {124 * 1024, 156 * 1024, 188 * 1024, 218 * 1024};
 constexpr size_t kContactLinkBytes = 11;
 
+// Diagnostics partial sums per block.
+constexpr int kDiagFields = 16;
+
+// Results read back through pinned memory (copies into pageable memory wait
+// for the stream each).
+struct HostReads {
+    Control control;
+    DevPayloadState payload;
+    double origin[3];
+    ContactDiagDev contact;
+    float4 nodes[16];
+    double applied[3];
+    int flag;
+    double partials[kDiagBlocks * kDiagFields];
+};
+
 struct StructureImpl {
     OwnedDefinition def;
     bool cluster_mode = false;
@@ -107,7 +124,13 @@ struct StructureImpl {
     int cur = 0;
     std::vector<float> inv_mass;  // by slot
     float4* d_force = nullptr;
-    float4* h_force = nullptr;    // pinned staging
+    float4* h_force = nullptr;    // pinned staging: the loads' upload, the states' download in pieces
+    size_t stage_bytes = 0;
+    HostReads* h_reads = nullptr;  // pinned: the small results a step or a query reads back
+    double* d_states = nullptr;    // node states in definition order, 9 doubles a node
+    uint32_t* d_slot_of_node = nullptr;
+    cudaEvent_t ev_stage[2] = {nullptr, nullptr};
+    mutable std::mutex reads;      // the staging is one caller's at a time
     uint4* d_tri = nullptr;
     uint32_t* d_tri_off = nullptr;
     uint32_t* d_tri_list = nullptr;
@@ -137,6 +160,7 @@ struct StructureImpl {
     // host mirror of the adapter state
     std::vector<swb_vec3> pending;
     std::vector<double> pressure;
+    bool pending_any = false;  // false: every pending load is zero
     bool forces_dirty = false;
     bool pressure_dirty = false;
     swb_vec3 last_applied{0, 0, 0};
@@ -181,6 +205,11 @@ struct StructureImpl {
     void fetch(std::vector<float4>& pos, std::vector<float4>& prev, std::vector<float4>& vel, DevPayloadState& pay,
                double origin[3]) const;
     void diagnostics(swb_diagnostics* out) const;
+    // its launch and copies on the state of buffer `buffer`, and, once the
+    // stream has run them, the result
+    void diagnostics_launch(int buffer) const;
+    void diagnostics_collect(swb_diagnostics* out) const;
+    void read_nodes(swb_node_state* out) const;
 };
 
 }  // namespace swb
