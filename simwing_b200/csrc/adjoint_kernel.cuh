@@ -468,16 +468,17 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_adjoint_kernel_t(con
     };
     const SweepArgs args{x_base, &flow, p.inv_dt, p.inv_dt2, nullptr, nullptr, nullptr, nullptr, nullptr};
     if (p.iterations > 0 && S > 0) fetch(p.iterations - 1, S - 1);
-    // The forward ran the line iteration beside its last two stages (neither
-    // touches a riser attachment node); the reverse of the line iteration runs
-    // beside the reverse of those two stages, on the same idle last warp of
-    // the suspension CTA: it arrives at the first reverse stage's barrier,
-    // runs, then waits at the second one's.
+    // The forward ran the line iteration beside its last stages (none touches
+    // a riser attachment node); the reverse of the line iteration runs beside
+    // the reverse of those stages, on the same idle last warp of the
+    // suspension CTA, which joins the others again at the barrier of the last
+    // of them it visits.
     const int line_stage = I.susp_cta >= 0 && !direct ? I.line_stage : -1;
-    const bool line_warp = line_stage >= 0 && owner && (tid >> 5) == static_cast<int>(blockDim.x >> 5) - 1;
+    const bool line_cta = line_stage >= 0 && owner;
+    const bool line_warp = line_cta && (tid >> 5) == static_cast<int>(blockDim.x >> 5) - 1;
     const int armer = blockDim.x >= 64 ? static_cast<int>(blockDim.x) - 33 : 0;
     const uint32_t slots = __ldg(I.patch_begin + p.ctas);
-    uint32_t sync_id = 1, phase = 0;  // phase: reverse iterations done
+    uint32_t phase = 0;  // reverse iterations done
     int it = p.iterations - 1;
     auto stage = [&]<int kKind>(int g) {
         const uint4 d = next_stage;
@@ -518,13 +519,14 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_adjoint_kernel_t(con
         }
         if (direct) {
             cluster.sync();
-        } else if (g == line_stage + 1 && line_warp) {
-            stage_arrive(sync_id);
-            line_reverse(pa, *ap, p.line_jac + static_cast<size_t>(it) * line_block, xb);
+        } else if (line_cta && g > line_stage) {
+            if (!line_warp)
+                stage_sync(2, blockDim.x - 32u);
+            else if (g == S - 1)
+                line_reverse(pa, *ap, p.line_jac + static_cast<size_t>(it) * line_block, xb);
         } else {
-            stage_sync(sync_id);
+            stage_sync(1, blockDim.x);
         }
-        sync_id ^= 3u;
         if (tid == armer) {
             if (barrier) flow_arm(flow.bar_base + barrier * 8u, flow.bytes[barrier]);
             if (g == S - 1 && phase > 0 && flow.home) flow_arm(flow.bar_base, flow.bytes[0]);

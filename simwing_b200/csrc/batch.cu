@@ -267,6 +267,9 @@ struct BatchImpl {
                     c.status = d_status + 2 * i;
                     c.recentre = m.def.has_suspension ? 1 : 0;
                     c.membrane_residual = m.d_mres[out];
+                    // a block narrower than the structure's own has no idle
+                    // warp for its line iteration
+                    if (P.threads < m.threads) c.line_stage = -1;
                     rec[(i * 3 + b) * 3 + role] = c;
                 }
         }

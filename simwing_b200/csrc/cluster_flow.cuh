@@ -38,13 +38,11 @@ __device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
     return remote;
 }
 
-// The CTA barrier between two stages, on one of two barrier resources so
-// that a warp that only arrives at one stage's barrier can wait at the next.
-__device__ __forceinline__ void stage_sync(uint32_t id) {
-    asm volatile("barrier.cta.sync.aligned %0, %1;" ::"r"(id), "r"(blockDim.x) : "memory");
-}
-__device__ __forceinline__ void stage_arrive(uint32_t id) {
-    asm volatile("barrier.cta.arrive.aligned %0, %1;" ::"r"(id), "r"(blockDim.x) : "memory");
+// The CTA barrier between two stages, for `threads` of the block: all, or all
+// but a warp that works across several stages (barriers of their own, so that
+// the two counts never meet on one).
+__device__ __forceinline__ void stage_sync(uint32_t id, uint32_t threads) {
+    asm volatile("barrier.cta.sync.aligned %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
 __device__ __forceinline__ void flow_arm(uint32_t bar, uint32_t bytes) {
@@ -92,14 +90,15 @@ __device__ __forceinline__ bool flow_test(uint32_t bar, uint32_t parity) {
     return done != 0;
 }
 
-__device__ __noinline__ void flow_wait_slow(const Flow& f, uint32_t bar, uint32_t parity) {
+// (by value: a reference would put the caller's Flow into local memory)
+__device__ __noinline__ void flow_wait_slow(uint32_t bar, uint32_t parity, int* dead, int* status, long long budget) {
     const long long start = clock64();
     while (!flow_test(bar, parity)) {
-        if (*static_cast<volatile int*>(f.dead)) return;
-        if (clock64() - start > f.budget) {
+        if (*static_cast<volatile int*>(dead)) return;
+        if (clock64() - start > budget) {
             // later waits of this CTA return at once, so the step ends
-            *static_cast<volatile int*>(f.dead) = 1;
-            atomicOr(f.status, kStatusSyncTimeout);
+            *static_cast<volatile int*>(dead) = 1;
+            atomicOr(status, kStatusSyncTimeout);
             return;
         }
     }
@@ -108,7 +107,7 @@ __device__ __noinline__ void flow_wait_slow(const Flow& f, uint32_t bar, uint32_
 // Waits for phase `iteration` of this CTA's barrier `index`.
 __device__ __forceinline__ void flow_wait(const Flow& f, uint32_t index, uint32_t iteration) {
     const uint32_t bar = f.bar_base + index * 8u;
-    if (!flow_test(bar, iteration & 1u)) flow_wait_slow(f, bar, iteration & 1u);
+    if (!flow_test(bar, iteration & 1u)) flow_wait_slow(bar, iteration & 1u, f.dead, f.status, f.budget);
 }
 
 // Sends a node where its word says (cluster_schedule.h, send_word).
@@ -119,6 +118,19 @@ __device__ __forceinline__ void flow_send(const Flow& f, uint32_t word, float4 v
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(to),
                  "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar)
                  : "memory");
+}
+
+// The same where `word` may be 0 (no send): predicated, so that a warp whose
+// lanes send different nodes of their records does not branch on each.
+__device__ __forceinline__ void flow_send_if(const Flow& f, uint32_t word, float4 v) {
+    const uint32_t rank = ((word >> 27) & 15u) + f.rank_base;
+    const uint32_t to = map_rank(f.x_base + (word & 0x3fffu) * 16u, rank);
+    const uint32_t bar = map_rank(f.bar_base + ((word >> 14) & 0x1fffu) * 8u, rank);
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.u32 p, %6, 0;\n"
+        " @p st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];\n}\n" ::"r"(to),
+        "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar), "r"(word)
+        : "memory");
 }
 
 // Direct schedules: the address of a foreign node.

@@ -18,7 +18,9 @@
 // fence stands between two stages.  With a cluster barrier after every stage
 // and foreign nodes read and written in place, the full wing (16 CTAs) took
 // 1.93 ms a step and a 9 x 9 patch (one CTA) 0.90 ms; handed over, in blocks
-// of up to 512 threads, 1.46 ms and 0.47 ms.
+// of up to 512 threads, 1.46 ms and 0.47 ms; with the pilot's line iteration
+// beside up to eight stages instead of two, and sends and stores predicated
+// instead of branched around, 1.33 ms.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -197,8 +199,7 @@ __device__ __forceinline__ void sweep_store(const SweepArgs& a, uint32_t slot, u
     }
     // (a node sent on comes back over this store before it is read here again)
     st_own(a.x_base + slot * 16u, v);
-    if constexpr (kMode == kHandOver)
-        if (word) flow_send(*a.flow, word, v);
+    if constexpr (kMode == kHandOver) flow_send_if(*a.flow, word, v);
 }
 
 template <int kKind, int kMode, bool kTape>
@@ -212,7 +213,14 @@ __device__ __forceinline__ void sweep_record(const SweepArgs& a, uint4 r, uint4 
             tape[i] = make_float4(A.x, A.y, A.z, l);
             tape[rtotal + i] = B;
         }
+        const float l0 = l;
         const bool ok = project_distance(A, B, __uint_as_float(r.z), __uint_as_float(r.w), l, a.inv_dt2);
+        if constexpr (kMode == kInside) {
+            st_own_if(ok, a.x_base + sa * 16u, A);
+            st_own_if(ok, a.x_base + sb * 16u, B);
+            *lam = ok ? l : l0;
+            return;
+        }
         if (!ok) {
             if constexpr (kMode != kHandOver) return;
             A = sweep_load<kMode>(a, sa, w.x);
@@ -231,7 +239,16 @@ __device__ __forceinline__ void sweep_record(const SweepArgs& a, uint4 r, uint4 
             tape[2 * rtotal + i] = C;
             tape[3 * rtotal + i] = D;
         }
+        const float l0 = l;
         const bool ok = project_dihedral(A, B, C, D, __uint_as_float(r.z), __uint_as_float(r.w), l, a.inv_dt2);
+        if constexpr (kMode == kInside) {
+            st_own_if(ok, a.x_base + sa * 16u, A);
+            st_own_if(ok, a.x_base + sb * 16u, B);
+            st_own_if(ok, a.x_base + sc * 16u, C);
+            st_own_if(ok, a.x_base + sd * 16u, D);
+            *lam = ok ? l : l0;
+            return;
+        }
         if (!ok) {
             if constexpr (kMode != kHandOver) return;
             A = sweep_load<kMode>(a, sa, w.x);
@@ -263,14 +280,15 @@ __device__ __forceinline__ void sweep_record(const SweepArgs& a, uint4 r, uint4 
     }
 }
 
-// Two distance-type records of a stage side by side on the CTA's own nodes
-// (a stage's records share no node): their two chains overlap, and the block
-// can be as narrow as the dihedral stages want it, with registers to spare
-// (full wing: 480 threads at 128 registers 1.46 ms a step, 736 threads at 80
-// registers, one record each, 1.65 ms).  `two`: there is a second one.
-template <bool kTape>
-__device__ __forceinline__ void sweep_distance_pair(const SweepArgs& a, uint4 r, uint4 s, bool two, float* lam_r,
-                                                    float* lam_s, uint32_t i, uint32_t j, float4* tape,
+// Two distance-type records of a stage side by side (a stage's records share
+// no node): their two chains overlap, and the block can be as narrow as the
+// dihedral stages want it, with registers to spare (full wing: 480 threads at
+// 128 registers 1.46 ms a step, 736 threads at 80 registers, one record each,
+// 1.65 ms).  The first may hand its nodes over (`w`), the second lies inside
+// the CTA's patch; `two`: there is a second one.
+template <int kMode, bool kTape>
+__device__ __forceinline__ void sweep_distance_pair(const SweepArgs& a, uint4 r, uint4 w, uint4 s, bool two,
+                                                    float* lam_r, float* lam_s, uint32_t i, uint32_t j, float4* tape,
                                                     uint32_t rtotal) {
     const uint32_t ra = a.x_base + (r.x & 0xffffu) * 16u, rb = a.x_base + (r.x >> 16) * 16u;
     const uint32_t sa = a.x_base + (s.x & 0xffffu) * 16u, sb = a.x_base + (s.x >> 16) * 16u;
@@ -285,18 +303,23 @@ __device__ __forceinline__ void sweep_distance_pair(const SweepArgs& a, uint4 r,
             tape[rtotal + j] = D;
         }
     }
+    const float lr0 = lr, ls0 = ls;
     const bool ok_r = project_distance(A, B, __uint_as_float(r.z), __uint_as_float(r.w), lr, a.inv_dt2);
+    if (kMode == kHandOver && !ok_r) {
+        A = ld_own(ra);
+        B = ld_own(rb);
+    }
+    st_own_if(kMode == kHandOver || ok_r, ra, A);
+    st_own_if(kMode == kHandOver || ok_r, rb, B);
+    if constexpr (kMode == kHandOver) {
+        flow_send_if(*a.flow, w.x, A);
+        flow_send_if(*a.flow, w.y, B);
+    }
+    *lam_r = ok_r ? lr : lr0;
     const bool ok_s = project_distance(C, D, __uint_as_float(s.z), __uint_as_float(s.w), ls, a.inv_dt2) && two;
-    if (ok_r) {
-        st_own(ra, A);
-        st_own(rb, B);
-        *lam_r = lr;
-    }
-    if (ok_s) {
-        st_own(sa, C);
-        st_own(sb, D);
-        *lam_s = ls;
-    }
+    st_own_if(ok_s, sa, C);
+    st_own_if(ok_s, sb, D);
+    if (two) *lam_s = ok_s ? ls : ls0;
 }
 
 // Records the pilot's inputs of a line iteration (or of the finish).
@@ -626,20 +649,20 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_kernel_t(const __gri
         stage_now = stage_next;
         stage_next = read_stage();
     }
-    // line iteration beside the last two stages: neither touches a
+    // line iteration beside the last stages: none of them touches a
     // suspension endpoint node, so running it there gives the same result as
     // running it after them.  The last warp of the suspension CTA (no record
-    // in either stage) arrives at the first stage's barrier, runs the line
-    // iteration, then waits at the second stage's; the next iteration's
-    // records read its writes after that.
+    // in any of them) runs it from the first on and joins the others again at
+    // the last one's barrier; between, their barriers go without it.  The
+    // next iteration's records read its writes after that.
     const bool susp = I.susp_cta >= 0;
-    const int line_stage = !kPacked && susp ? I.line_stage : -1;
-    const bool line_warp = line_stage >= 0 && owner && (tid >> 5) == static_cast<int>(blockDim.x >> 5) - 1;
+    const int line_stage = susp && !stages_c ? I.line_stage : -1;
+    const bool line_cta = line_stage >= 0 && owner;
+    const bool line_warp = line_cta && (tid >> 5) == static_cast<int>(blockDim.x >> 5) - 1;
     // the thread that arms the barriers again: not of the last warp, which
     // may run the line iteration, nor (with two warps or more to spare) of
     // the first ones, which have the boundary records
     const int armer = blockDim.x >= 64 ? static_cast<int>(blockDim.x) - 33 : 0;
-    uint32_t sync_id = 1;
     int it = 0;
     // One stage: its records, then the CTA barrier (a cluster barrier in a
     // cluster with a direct schedule).
@@ -662,13 +685,20 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_kernel_t(const __gri
                 if (utid < d.y) sweep_record<kKind, kDirect, kTape>(args, r, w, lam_i, i - kind0, tape, rtotal);
             } else {
                 if (barrier) flow_wait(flow, barrier, static_cast<uint32_t>(it));
-                if (utid < d.y) sweep_record<kKind, kHandOver, kTape>(args, r, w, lam_i, i - kind0, tape, rtotal);
+                if (utid < d.y) {
+                    if constexpr (kKind == 0)
+                        sweep_distance_pair<kHandOver, kTape>(args, r, w, r2, two && edges <= width, lam_i, lam_i + width,
+                                                              i, i + width, tape, rtotal);
+                    else
+                        sweep_record<kKind, kHandOver, kTape>(args, r, w, lam_i, i - kind0, tape, rtotal);
+                }
             }
-            if (two && edges <= width)
+            if ((kKind != 0 || direct) && two && edges <= width)
                 sweep_record<kKind, kInside, kTape>(args, r2, w, lam_i + kLam * width, i + width - kind0, tape, rtotal);
         } else if (utid < d.y) {
             if constexpr (kKind == 0) {
-                sweep_distance_pair<kTape>(args, r, r2, two, lam_i, lam_i + width, i, i + width, tape, rtotal);
+                sweep_distance_pair<kInside, kTape>(args, r, w, r2, two, lam_i, lam_i + width, i, i + width, tape,
+                                                    rtotal);
             } else {
                 sweep_record<kKind, kInside, kTape>(args, r, w, lam_i, i - kind0, tape, rtotal);
                 if (two)
@@ -689,17 +719,19 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_kernel_t(const __gri
         }
         if (stages_c) {
             cluster.sync();
-        } else if (g == line_stage && line_warp) {
-            stage_arrive(sync_id);
-            if ((tid & 31) == 0) {
-                if constexpr (kTape) tape_pilot(p.tape.line[it], pay, *p.tape.pilot, x, nullptr);
-                line_iteration(pdef, pay, x, p.dt, I.status);
+        } else if (line_cta && g >= line_stage && g + 1 < S) {
+            if (!line_warp) {
+                stage_sync(2, width - 32u);
+            } else if (g == line_stage) {
+                if ((tid & 31) == 0) {
+                    if constexpr (kTape) tape_pilot(p.tape.line[it], pay, *p.tape.pilot, x, nullptr);
+                    line_iteration(pdef, pay, x, p.dt, I.status);
+                }
+                __syncwarp();
             }
-            __syncwarp();
         } else {
-            stage_sync(sync_id);
+            stage_sync(1, width);
         }
-        sync_id ^= 3u;
         if (tid == armer) {
             if (barrier) flow_arm(flow.bar_base + barrier * 8u, flow.bytes[barrier]);
             if (g == 0 && it > 0 && flow.home) flow_arm(flow.bar_base, flow.bytes[0]);

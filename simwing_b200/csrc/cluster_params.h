@@ -210,10 +210,9 @@ struct ClusterInstance {
     double* origin_out;
     int* status;
     int recentre;
-    // First of the two stages beside which the line iteration runs (on the
-    // last warp of the suspension CTA, which has no record in either), or -1:
-    // the line iteration then follows the iteration's stages behind a
-    // cluster barrier.  Single-structure launches only.
+    // First of the iteration's last stages beside which the line iteration
+    // runs (on the last warp of the suspension CTA, which has no record in any
+    // of them), or -1: the line iteration then follows the stages.
     int line_stage;
     // 1: the momentum guard of free structures runs (no suspension, no
     // contact, bending or membranes present, every node free:

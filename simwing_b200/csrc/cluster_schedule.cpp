@@ -790,13 +790,15 @@ bool build_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_t
         direct = true;
     }
 
-    // line iteration window: the last two stages of the iteration, when
-    // neither touches a suspension endpoint node
-    if (S.susp_cta >= 0 && !(split && ctas > 1)) {
+    // line iteration window: the last stages of the iteration that touch no
+    // suspension endpoint node, two at least
+    if (S.susp_cta >= 0 && !(split && ctas > 1) && !direct) {
         const int Sg = total_stages(S);
-        if (Sg >= 2 && !direct && !stage_touches(d, S, attached, Sg - 2) && !stage_touches(d, S, attached, Sg - 1)) {
-            S.line_stage = Sg - 2;
-            for (int g = Sg - 2; g < Sg; ++g) {
+        int first = Sg;
+        while (first > 0 && Sg - first < kLineWindow && !stage_touches(d, S, attached, first - 1)) --first;
+        if (Sg - first >= 2) {
+            S.line_stage = first;
+            for (int g = first; g < Sg; ++g) {
                 int k, s;
                 global_stage(S, g, k, s);
                 const ClusterKind& K = S.kinds[k];
@@ -946,10 +948,11 @@ void verify_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_
     }
     if (S.line_stage >= 0) {
         const int Sg = total_stages(S);
-        if (S.susp_cta < 0 || S.line_stage != Sg - 2) fail("line iteration window position");
+        if (S.susp_cta < 0 || S.line_stage > Sg - 2 || S.line_stage < Sg - kLineWindow)
+            fail("line iteration window position");
         std::vector<uint8_t> attached(N, 0);
         for (uint32_t n : suspension_nodes) attached[n] = 1;
-        for (int g = Sg - 2; g < Sg; ++g) {
+        for (int g = S.line_stage; g < Sg; ++g) {
             int k, s;
             global_stage(S, g, k, s);
             if (stage_touches(d, S, attached, g)) fail("line iteration window touches a suspension node");

@@ -127,13 +127,13 @@ struct ClusterSchedule {
     std::vector<uint32_t> seam_offsets;  // [ctas * (seam_stages + 1)]
     std::vector<uint32_t> seam_ab;
     int susp_cta = -1;
-    // Line iteration window (classic stages only): when the last two stages
-    // of an iteration touch no suspension endpoint node, the iteration's line
-    // iteration runs beside them on a warp of the suspension CTA that has no
-    // record in either, instead of after them behind a barrier of its own.
-    // line_stage = the first of the two (global stage index: distance stages
-    // then dihedral stages), -1 without a window; line_owner_records = the
-    // suspension CTA's larger record count of the two.
+    // Line iteration window (classic stages only): the last stages of an
+    // iteration, two to kLineWindow of them, that touch no suspension endpoint
+    // node.  The iteration's line iteration runs beside them on the last warp
+    // of the suspension CTA, which has no record in any, instead of after
+    // them.  line_stage = the first of them (global stage index), -1 without
+    // a window; line_owner_records = the suspension CTA's largest record count
+    // in the window.
     int line_stage = -1;
     uint32_t line_owner_records = 0;
     std::vector<uint64_t> distance_order, dihedral_order, membrane_order;
@@ -198,6 +198,10 @@ struct ClusterLayout {
     uint32_t velocity = 0, stages = 0, barriers = 0, bytes = 0, total = 0;
 };
 ClusterLayout layout_of(const ClusterSchedule& s);
+
+// Stages a line iteration may run beside: one takes about 5 us, a stage of a
+// wing 0.5 to 1 us.
+constexpr int kLineWindow = 8;
 
 // Returns false (and leaves `out` empty) when the mesh does not fit one
 // cluster of `ctas` CTAs (a patch over kClusterPatchNodes nodes).  The

@@ -149,6 +149,12 @@ __device__ __forceinline__ void st_own(uint32_t addr, float4 v) {
     asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w));
 }
 
+// The store where `ok`, predicated (a branch around it costs more).
+__device__ __forceinline__ void st_own_if(bool ok, uint32_t addr, float4 v) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %5, 0;\n @p st.shared.v4.f32 [%0], {%1, %2, %3, %4};\n}\n" ::"r"(addr),
+                 "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(static_cast<uint32_t>(ok)));
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned int count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
