@@ -350,7 +350,7 @@ struct RolloutImpl {
         const int K = std::min(interval, steps - c * interval);
         copy_state(ck[c], sg[0]);
         cudaLaunchAttribute attr[1];
-        const cudaLaunchConfig_t cfg = config(S->cluster_smem, S->threads, attr);
+        const cudaLaunchConfig_t cfg = config(S->step_smem(), S->threads, attr);
         for (int k = 0; k < K; ++k) {
             const ClusterParams cp = step_params(k, with_tape ? &tape[k] : nullptr);
             cuda_check(with_tape ? tape_kernel_launch(cfg, cp) : plain_cluster_launch(cfg, cp), "rollout step");

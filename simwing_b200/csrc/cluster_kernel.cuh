@@ -783,7 +783,12 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_kernel_t(const __gri
                     line_tape = p.tape.line_in + static_cast<size_t>(it) * p.tape.line_cap * 4;
             }
             cluster.sync();
-            if (me == 0) line_project(*lines, line_addr, line_tape);
+            if (me == 0) {
+                if (lines->smem_near != ~0u)
+                    line_project_near(*lines, line_addr, smem + lines->smem_near, line_tape);
+                else
+                    line_project(*lines, line_addr, line_tape);
+            }
             cluster.sync();
         }
         if (p.ground) {

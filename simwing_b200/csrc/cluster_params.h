@@ -167,7 +167,23 @@ struct LineContactDev {
     uint32_t* pred;                    // [capacity][4] per node the latest earlier pair with it (~0u: none)
     uint32_t* level_off;               // [capacity + 1] each level's first place in `order`
     uint32_t* count;                   // [2] candidate pairs of the step, their level count
+    // the cable nodes as rank 0 gathers them for the projections: home
+    // references, the segments' ends among them (a | b << 16), the ordered
+    // candidates' four (a | b << 16, c | d << 16), and the place in shared
+    // memory (byte offset; ~0u: no room, the nodes are projected in place)
+    uint32_t nodes;
+    const uint32_t* node_ref;          // [nodes]
+    const uint32_t* seg_near;          // [segments]
+    uint2* cand_near;                  // [capacity]
+    uint32_t smem_near;
 };
+
+// Shared memory of the gathered cable nodes: the nodes, a mark per node that
+// a projection has moved it, a bit per candidate that starts out too near.
+constexpr uint32_t kLineCandidates = 1u << 16;
+inline uint32_t line_near_bytes(uint32_t nodes) {
+    return nodes * 16u + ((nodes + 15u) & ~15u) + kLineCandidates / 8u;
+}
 
 // The hand-overs of a sweep (ClusterFlow, cluster_schedule.h).
 struct ClusterFlowDev {

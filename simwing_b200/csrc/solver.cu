@@ -479,8 +479,37 @@ void StructureImpl::setup_line_contact() {
         nodes[i] = make_uint2(static_cast<uint32_t>(segs[i].first), static_cast<uint32_t>(segs[i].second));
     }
     LineContactDev L{};
+    // the cable nodes, numbered, and the segments' ends among them
+    std::vector<uint32_t> near(2 * segs.size()), node_ref;
+    {
+        std::vector<uint64_t> ids;
+        for (const auto& g : segs) {
+            ids.push_back(g.first);
+            ids.push_back(g.second);
+        }
+        std::sort(ids.begin(), ids.end());
+        ids.erase(std::unique(ids.begin(), ids.end()), ids.end());
+        auto at = [&](uint64_t node) {
+            return static_cast<uint32_t>(std::lower_bound(ids.begin(), ids.end(), node) - ids.begin());
+        };
+        near.resize(segs.size());
+        for (size_t i = 0; i < segs.size(); ++i)
+            near[i] = (at(segs[i].first) & 0xffffu) | at(segs[i].second) << 16;
+        for (uint64_t id : ids) node_ref.push_back(ref(id));
+    }
     L.segments = static_cast<uint32_t>(segs.size());
-    L.capacity = 1u << 16;
+    L.capacity = kLineCandidates;
+    L.nodes = static_cast<uint32_t>(node_ref.size());
+    L.node_ref = dupload(owned, node_ref, stream);
+    L.seg_near = dupload(owned, near, stream);
+    L.cand_near = dalloc<uint2>(owned, L.capacity);
+    // gathered beside the patch where there is room
+    line_smem = 0;
+    L.smem_near = ~0u;
+    if (L.nodes < 65536 && cluster_smem + line_near_bytes(L.nodes) <= smem_cap) {
+        L.smem_near = cluster_smem;
+        line_smem = line_near_bytes(L.nodes);
+    }
     L.seg = dupload(owned, seg, stream);
     L.seg_nodes = dupload(owned, nodes, stream);
     L.box = dalloc<float4>(owned, 2 * std::max<size_t>(segs.size(), 1));
@@ -1074,7 +1103,7 @@ void StructureImpl::launch_substep(const swb_step_settings& st, int in, int out,
         attr[1].val.cooperative = 1;
         cfg.gridDim = dim3(G * (1 + contact_helpers));
         cfg.blockDim = dim3(threads);
-        cfg.dynamicSmemBytes = cluster_smem;
+        cfg.dynamicSmemBytes = step_smem();
         cfg.stream = stream;
         cfg.attrs = attr;
         cfg.numAttrs = contact_helpers > 0 ? 2 : 1;

@@ -100,6 +100,8 @@ struct StructureImpl {
     ClusterInstance cluster_base{};
     ClusterInstance* d_instances = nullptr;
     uint32_t cluster_smem = 0;
+    uint32_t line_smem = 0;    // the gathered cable nodes of line-line contact, after it
+    uint32_t step_smem() const { return cluster_smem + (line_contact ? line_smem : 0); }
     uint64_t fingerprint = 0;
     int device = -1;
     int sm_count = 0;
