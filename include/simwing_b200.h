@@ -300,8 +300,8 @@ typedef struct swb_wrench {
 /* ------------------------------------------------------------------------ */
 /* Two device schedules exist.  The cluster schedule (default when the mesh
  * fits: at most 16 x 4096 nodes and the shared-memory budget) keeps every
- * node in the distributed shared memory of one thread-block cluster and
- * separates colour stages with cluster barriers.  The grid schedule spreads
+ * node in the distributed shared memory of one thread-block cluster, whose
+ * CTAs hand the nodes they share from one to the next.  The grid schedule spreads
  * patches over a persistent cooperative grid with device-wide barriers and
  * serves meshes that do not fit one cluster. */
 typedef struct swb_solver_options {
@@ -323,9 +323,8 @@ enum {
     SWB_OPT_GRID = 1u << 2,        /* force the grid schedule                */
     SWB_OPT_SPLIT_STAGES = 1u << 3, /* cluster schedule with split stages:
                                       stages of records that touch only the
-                                      executing CTA's patch behind CTA
-                                      barriers, cluster barriers after the
-                                      stages of records that span CTAs       */
+                                      executing CTA's patch first, the stages
+                                      of records that span CTAs after them   */
     SWB_OPT_AUTOTUNE = 1u << 4,    /* swb_structure_create builds the cluster
                                       schedule for several block sizes (the
                                       widest stage, 512, 768 threads), with
@@ -562,7 +561,8 @@ typedef struct swb_schedule_report {
     uint64_t level_constraints[4];       /* distance+dihedral per level      */
     uint64_t global_constraints;
     int32_t cluster_ctas;                /* 0 = grid schedule                */
-    int32_t cluster_barriers_per_iteration;
+    int32_t cluster_barriers_per_iteration; /* stages whose records may span
+                                      CTAs, after which nodes change hands    */
 } swb_schedule_report;
 /* The autotuner's candidates (SWB_OPT_AUTOTUNE) and its choice; zero
  * candidates when the structure was not tuned.  No reference counterpart. */

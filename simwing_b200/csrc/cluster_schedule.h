@@ -169,8 +169,8 @@ inline void global_stage(const ClusterSchedule& s, int g, int& kind, int& local)
     }
 }
 
-// Cluster barriers per constraint iteration (stages followed by one, plus
-// the suspension stage unless the line iteration runs beside two stages).
+// Stages of an iteration whose records may span CTAs (after which nodes
+// change hands), plus the line iteration where it follows the stages.
 inline int cluster_barriers_per_iteration(const ClusterSchedule& s) {
     int n = s.susp_cta >= 0 && s.line_stage < 0 ? 1 : 0;
     for (const ClusterKind& k : s.kinds)
