@@ -823,7 +823,7 @@ struct __align__(128) ContactWork {
     uint32_t addr[4];
     float inv[4];
     double lambda;      // the warm start
-    uint32_t fc_flags;  // fc | the warm start entry's flags << 8
+    uint32_t fc_flags;  // fc | the warm start entry's flags << 8 (the failure's detail code when fc = 0)
     uint32_t cand;      // candidate index
     double2 pad;
 };
@@ -835,21 +835,20 @@ __device__ __forceinline__ ContactWork* contact_work(const ContactDev& C) {
 
 // The work record of hit `h` (candidate i): the checks and the orientation
 // the projection starts with (contact.cpp:1318-1351), and its nodes'
-// addresses.
+// addresses.  A check that fails is reported by the projection in its turn:
+// the status word must not change while the cluster still branches on it.
 static __device__ __noinline__ void prepare_work(const ContactCtx& c, uint32_t h, uint32_t i) {
     const ContactDev& C = *c.C;
     ContactQuery& Q = C.query[i];
     const ContactEntry& e = C.cand_entry[i];
-    uint32_t live = 0;
+    uint32_t fc_flags = Q.fc | e.flags << 8;
     D3 normal = d3_of(Q.normal);
     if (!Q.certified) {
-        contact_fail_at(C, c.status, kContactGeometry, C.cand[i]);
+        fc_flags = static_cast<uint32_t>(kContactGeometry) << 8;
     } else {
         if (contact::dot(normal, d3_of(Q.ccd_normal)) < 0.0) normal = -normal;
         if (!contact::finite3(normal) || fabs(contact::norm2(normal) - 1.0) > 1.0e-8)
-            contact_fail_at(C, c.status, kContactNormal, C.cand[i]);
-        else
-            live = Q.fc;
+            fc_flags = static_cast<uint32_t>(kContactNormal) << 8;
     }
     const int fc = static_cast<int>(Q.fc);
     ContactWork W;
@@ -865,7 +864,7 @@ static __device__ __noinline__ void prepare_work(const ContactCtx& c, uint32_t h
     W.normal_xy = make_double2(normal.x, normal.y);
     W.normal_z_eff = make_double2(normal.z, Q.eff);
     W.lambda = e.lambda;
-    W.fc_flags = live | e.flags << 8;
+    W.fc_flags = fc_flags;
     W.cand = i;
     W.pad = make_double2(0.0, 0.0);
     contact_work(C)[h] = W;
@@ -890,7 +889,10 @@ __device__ __forceinline__ void project_one(const ContactWork& W, const ProjectC
     const uint32_t ff = W.fc_flags, cand = W.cand;
     const float inv = W.inv[g.node];
     const uint32_t fc = ff & 0xffu, flags = ff >> 8;
-    if (fc == 0) return;
+    if (fc == 0) {
+        if (g.lane == 0) contact_fail_at(*pc.C, pc.status, static_cast<int>(flags), pc.C->cand[cand]);
+        return;
+    }
     const uint32_t addr = home + 4u * g.comp;
     const float x = ld_component(addr);
     const double w[4] = {w01.x, w01.y, w23.x, w23.y};
@@ -991,7 +993,9 @@ __device__ __noinline__ void contact_project(const ContactCtx& c, cooperative_gr
                 if (C.mark_a[i + 1] != C.mark_a[i]) C.hit[C.mark_a[i]] = i;
     }
     cluster.sync();
-    if (!contact_failed(c.status)) {  // uniform: read after the barrier
+    // uniform: read after the barrier, and written next by rank 0's rounds,
+    // behind cluster_order's barriers
+    if (!contact_failed(c.status)) {
         const uint32_t hits = C.mark_a[count];
         // the work records of the candidates in contact (read by rank 0's
         // rounds after cluster_order's barriers)
