@@ -360,6 +360,7 @@ struct RolloutImpl {
 
     void check_status() {
         std::string message;
+        const std::lock_guard<std::mutex> lock(S->reads);
         const swb_status st = S->read_status(message);
         if (st != SWB_OK) raise(st, "rollout: " + message);
     }

@@ -26,8 +26,15 @@ struct swb_coupling {
     int* d_flag = nullptr;          // 1: a non-finite load
     std::vector<double> pending_host;  // staging of the pending loads
     std::vector<void*> owned;
+    // pinned: what a call reads back beside the step's own results
+    struct Results {
+        double applied[3];
+        int flag;
+    };
+    Results* results = nullptr;
     ~swb_coupling() {
         for (void* p : owned) cudaFree(p);
+        if (results) cudaFreeHost(results);
     }
 };
 
@@ -138,9 +145,9 @@ swb_status advance(swb_coupling* c, const double* a, const double* b, double sca
                                                                         c->d_pending, a, b, scale, endpoints,
                                                                         S.d_force, total64, c->d_flag);
         cuda_check(cudaGetLastError(), "gather_loads_kernel");
-        cuda_check(cudaMemcpyAsync(&S.h_reads->flag, c->d_flag, sizeof(int), cudaMemcpyDeviceToHost, S.stream), "read");
+        cuda_check(cudaMemcpyAsync(&c->results->flag, c->d_flag, sizeof(int), cudaMemcpyDeviceToHost, S.stream), "read");
         cuda_check(cudaStreamSynchronize(S.stream), "gather");
-        if (S.h_reads->flag) {
+        if (c->results->flag) {
             S.forces_dirty = true;  // the device buffer no longer holds the pending loads
             raise(SWB_INVALID_ARGUMENT, "time-integrated transfer has invalid nodal bindings or non-finite loads");
         }
@@ -149,8 +156,8 @@ swb_status advance(swb_coupling* c, const double* a, const double* b, double sca
         applied_total_kernel<<<1, 1024, 0, S.stream>>>(S.def.nodes.size(), c->d_items + c->bindings, total64,
                                                        c->d_applied);
         cuda_check(cudaGetLastError(), "applied_total_kernel");
-        cuda_check(cudaMemcpyAsync(S.h_reads->applied, c->d_applied, sizeof(S.h_reads->applied), cudaMemcpyDeviceToHost,
-                                   S.stream), "read");
+        cuda_check(cudaMemcpyAsync(c->results->applied, c->d_applied, sizeof(c->results->applied),
+                                   cudaMemcpyDeviceToHost, S.stream), "read");
         S.device_forces = true;
         try {
             S.step(*settings, 1, out);
@@ -160,7 +167,7 @@ swb_status advance(swb_coupling* c, const double* a, const double* b, double sca
             throw;
         }
         S.device_forces = false;
-        const swb_vec3 applied{S.h_reads->applied[0], S.h_reads->applied[1], S.h_reads->applied[2]};
+        const swb_vec3 applied{c->results->applied[0], c->results->applied[1], c->results->applied[2]};
         S.last_applied = applied;
         S.forces_dirty = true;  // the buffer holds this call's loads; pending is empty again
         if (out) out->last_applied_external_force = applied;
@@ -200,6 +207,7 @@ swb_status swb_coupling_create(swb_structure* structure, const uint64_t* structu
         c->d_pending = alloc<double>(c->owned, 3 * N);
         c->d_applied = alloc<double>(c->owned, 3);
         c->d_flag = alloc<int>(c->owned, 1);
+        cuda_check(cudaMallocHost(&c->results, sizeof(*c->results)), "cudaMallocHost");
         cuda_check(cudaMemcpy(c->d_offsets, counts.data(), (N + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice),
                    "upload");
         cuda_check(cudaMemcpy(c->d_items, items.data(), items.size() * sizeof(uint32_t), cudaMemcpyHostToDevice),

@@ -356,10 +356,13 @@ void StructureImpl::build(const swb_structure_definition& definition, const swb_
     }
     d_force = dalloc<float4>(owned, N);
     cuda_check(cudaMemsetAsync(d_force, 0, N * sizeof(float4), stream), "memset");
-    // pinned: the staging, at least 64 KB, and the small results behind it
-    stage_bytes = (std::max<size_t>(N * sizeof(float4), 64 * 1024) + 511) & ~size_t{511};
-    cuda_check(cudaMallocHost(&h_force, stage_bytes + sizeof(HostReads)), "cudaMallocHost");
-    h_reads = reinterpret_cast<HostReads*>(reinterpret_cast<unsigned char*>(h_force) + stage_bytes);
+    // pinned: the loads' upload, the states' download (at least 64 KB) and the
+    // small results
+    const size_t load_bytes = (N * sizeof(float4) + 511) & ~size_t{511};
+    stage_bytes = std::max<size_t>(load_bytes, 64 * 1024);
+    cuda_check(cudaMallocHost(&h_force, load_bytes + stage_bytes + sizeof(HostReads)), "cudaMallocHost");
+    h_stage = reinterpret_cast<unsigned char*>(h_force) + load_bytes;
+    h_reads = reinterpret_cast<HostReads*>(h_stage + stage_bytes);
     d_states = dalloc<double>(owned, 9 * N);
     d_slot_of_node = dupload(owned, slot_of_node, stream);
     for (cudaEvent_t& e : ev_stage) cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
@@ -1456,17 +1459,16 @@ void StructureImpl::read_nodes(swb_node_state* out) const {
     cuda_check(cudaGetLastError(), "gather_states_kernel");
     const size_t total = N * sizeof(swb_node_state), piece = (stage_bytes / 2) & ~size_t{255};
     const size_t pieces = (total + piece - 1) / piece;
-    unsigned char* stage = reinterpret_cast<unsigned char*>(h_force);
     auto bytes_of = [&](size_t k) { return std::min(piece, total - k * piece); };
     auto issue = [&](size_t k) {
-        cuda_check(cudaMemcpyAsync(stage + (k & 1) * piece, reinterpret_cast<const unsigned char*>(d_states) + k * piece,
+        cuda_check(cudaMemcpyAsync(h_stage + (k & 1) * piece, reinterpret_cast<const unsigned char*>(d_states) + k * piece,
                                    bytes_of(k), cudaMemcpyDeviceToHost, stream), "read");
         cuda_check(cudaEventRecord(ev_stage[k & 1], stream), "event");
     };
     for (size_t k = 0; k < std::min<size_t>(2, pieces); ++k) issue(k);
     for (size_t k = 0; k < pieces; ++k) {
         cuda_check(cudaEventSynchronize(ev_stage[k & 1]), "read");
-        std::memcpy(reinterpret_cast<unsigned char*>(out) + k * piece, stage + (k & 1) * piece, bytes_of(k));
+        std::memcpy(reinterpret_cast<unsigned char*>(out) + k * piece, h_stage + (k & 1) * piece, bytes_of(k));
         if (k + 2 < pieces) issue(k + 2);
     }
 }
@@ -1584,6 +1586,7 @@ void swb_default_solver_options(swb_solver_options* out) {
 }
 
 double StructureImpl::time_trial(const swb_step_settings& st, int warm, int reps) {
+    const std::lock_guard<std::mutex> lock(reads);
     cuda_check(cudaSetDevice(device), "cudaSetDevice");
     if (pressure_dirty) upload_pressure();
     if (forces_dirty && !device_forces) upload_forces();

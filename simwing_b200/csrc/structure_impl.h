@@ -74,15 +74,13 @@ constexpr size_t kContactLinkBytes = 11;
 constexpr int kDiagFields = 16;
 
 // Results read back through pinned memory (copies into pageable memory wait
-// for the stream each).
+// for the stream each), under StructureImpl::reads.
 struct HostReads {
     Control control;
     DevPayloadState payload;
     double origin[3];
     ContactDiagDev contact;
     float4 nodes[16];
-    double applied[3];
-    int flag;
     double partials[kDiagBlocks * kDiagFields];
 };
 
@@ -126,13 +124,16 @@ struct StructureImpl {
     int cur = 0;
     std::vector<float> inv_mass;  // by slot
     float4* d_force = nullptr;
-    float4* h_force = nullptr;    // pinned staging: the loads' upload, the states' download in pieces
+    float4* h_force = nullptr;    // pinned staging of the loads' upload
+    // pinned staging of the states' download, in pieces: apart from the
+    // loads', which a rollout or a batch uploads while another thread reads
+    unsigned char* h_stage = nullptr;
     size_t stage_bytes = 0;
     HostReads* h_reads = nullptr;  // pinned: the small results a step or a query reads back
     double* d_states = nullptr;    // node states in definition order, 9 doubles a node
     uint32_t* d_slot_of_node = nullptr;
     cudaEvent_t ev_stage[2] = {nullptr, nullptr};
-    mutable std::mutex reads;      // the staging is one caller's at a time
+    mutable std::mutex reads;      // h_stage and h_reads are one caller's at a time
     uint4* d_tri = nullptr;
     uint32_t* d_tri_off = nullptr;
     uint32_t* d_tri_list = nullptr;
