@@ -477,6 +477,9 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_adjoint_kernel_t(con
     const bool line_cta = line_stage >= 0 && owner;
     const bool line_warp = line_cta && (tid >> 5) == static_cast<int>(blockDim.x >> 5) - 1;
     const int armer = blockDim.x >= 64 ? static_cast<int>(blockDim.x) - 33 : 0;
+    // the first stage visited whose barrier the whole block takes: after it
+    // every thread is past its wait for the last home-coming
+    const int home_stage = line_cta ? line_stage : S - 1;
     const uint32_t slots = __ldg(I.patch_begin + p.ctas);
     uint32_t phase = 0;  // reverse iterations done
     int it = p.iterations - 1;
@@ -529,7 +532,7 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_adjoint_kernel_t(con
         }
         if (tid == armer) {
             if (barrier) flow_arm(flow.bar_base + barrier * 8u, flow.bytes[barrier]);
-            if (g == S - 1 && phase > 0 && flow.home) flow_arm(flow.bar_base, flow.bytes[0]);
+            if (g == home_stage && phase > 0 && flow.home) flow_arm(flow.bar_base, flow.bytes[0]);
         }
     };
     for (; it >= 0; --it, ++phase) {

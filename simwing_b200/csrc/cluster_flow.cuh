@@ -7,8 +7,9 @@
 //
 // A barrier's phase p is iteration p (reverse sweeps count their own): it
 // is armed again for the next iteration only after the CTA barrier that
-// closes the receiving stage, when every thread has passed its wait.  The
-// next iteration's first nodes may be counted before that (a transaction
+// closes the receiving stage (for the nodes that come home, the next
+// iteration's first barrier of the whole block), when every thread has passed
+// its wait.  The next iteration's first nodes may be counted before that (a transaction
 // count may run ahead of its arming); the phase cannot end before the
 // arming, which is its only arrival.  A node is not overwritten before its
 // reader is done: its next value exists only after the reader's result.

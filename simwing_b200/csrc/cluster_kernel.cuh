@@ -663,6 +663,9 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_kernel_t(const __gri
     // may run the line iteration, nor (with two warps or more to spare) of
     // the first ones, which have the boundary records
     const int armer = blockDim.x >= 64 ? static_cast<int>(blockDim.x) - 33 : 0;
+    // the stage whose barrier is the iteration's first that the whole block
+    // takes: after it every thread is past its wait for the last home-coming
+    const int home_stage = line_cta && line_stage == 0 ? S - 1 : 0;
     int it = 0;
     // One stage: its records, then the CTA barrier (a cluster barrier in a
     // cluster with a direct schedule).
@@ -734,7 +737,7 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_kernel_t(const __gri
         }
         if (tid == armer) {
             if (barrier) flow_arm(flow.bar_base + barrier * 8u, flow.bytes[barrier]);
-            if (g == 0 && it > 0 && flow.home) flow_arm(flow.bar_base, flow.bytes[0]);
+            if (g == home_stage && it > 0 && flow.home) flow_arm(flow.bar_base, flow.bytes[0]);
         }
     };
     // load-path cable sweeps (soft_body.cpp:1288-1317): a quarter of the
