@@ -38,7 +38,7 @@ typedef enum swb_status {
     SWB_SUSPENSION_ERROR = 3,   /* softwing::SuspensionError                */
     SWB_CONTACT_ERROR = 4,      /* softwing::ContactStepError               */
     SWB_NON_FINITE = 5,         /* device detected NaN/Inf in the trial step */
-    SWB_SYNC_TIMEOUT = 6,       /* a bounded device-wide barrier gave up     */
+    SWB_SYNC_TIMEOUT = 6,       /* a bounded barrier or wait gave up         */
     SWB_CUDA_ERROR = 7,         /* CUDA runtime failure                      */
     SWB_UNSUPPORTED = 8,        /* feature not available in this build       */
     SWB_OUT_OF_MEMORY = 9
@@ -484,6 +484,14 @@ typedef struct swb_line_contact {
     uint32_t reserved;
 } swb_line_contact;
 swb_status swb_structure_set_line_contact(swb_structure* structure, const swb_line_contact* contact);
+
+/* Limit, in GPU cycles, of one wait of the cluster schedule for nodes handed
+ * over from another CTA (0 = default, ~2 s).  A step or rollout in which one
+ * runs out fails with SWB_SYNC_TIMEOUT and leaves the state as it was.
+ * held_cta >= 0 makes that happen, for tests: the CTA leaves its sweep out, and
+ * the waits for its nodes run out (-1: none; no effect where the schedule hands
+ * no nodes over).  No reference counterpart. */
+swb_status swb_structure_set_wait_limit(swb_structure* structure, int64_t cycles, int32_t held_cta);
 
 /* The device forms of the step's two short math functions on host arrays
  * (no counterpart in the reference; for checking them on the GPU they run

@@ -678,6 +678,11 @@ class Structure:
         lc = abi.LineContact(float(radius), float(margin), 1 if enabled else 0, 0)
         _check(self._lib.swb_structure_set_line_contact(self._h, C.byref(lc)))
 
+    def set_wait_limit(self, cycles: int = 0, held_cta: int = -1) -> None:
+        """Cycles a wait for handed-over nodes may take, 0: the default; a CTA
+        whose nodes never come, for tests (swb_structure_set_wait_limit)."""
+        _check(self._lib.swb_structure_set_wait_limit(self._h, int(cycles), int(held_cta)))
+
     def step(self, settings: abi.StepSettings | None = None, diagnostics: bool = True):
         s = settings if settings is not None else StepSettings()
         d = abi.Diagnostics()

@@ -376,6 +376,7 @@ _PROTOTYPES = {
     "swb_structure_set_uniform_pressure": (C.c_int, [C.c_void_p, C.c_double]),
     "swb_structure_set_ground": (C.c_int, [C.c_void_p, C.c_void_p]),
     "swb_structure_set_line_contact": (C.c_int, [C.c_void_p, C.c_void_p]),
+    "swb_structure_set_wait_limit": (C.c_int, [C.c_void_p, C.c_int64, C.c_int32]),
     "swb_structure_step": (C.c_int, [C.c_void_p, P(StepSettings), P(Diagnostics)]),
     "swb_structure_step_many": (C.c_int, [C.c_void_p, P(StepSettings), C.c_int32, P(Diagnostics)]),
     "swb_structure_diagnostics": (C.c_int, [C.c_void_p, P(Diagnostics)]),

@@ -246,7 +246,6 @@ struct RolloutImpl {
         base.flow.smem_stages = offsets.smem_stages;
         base.flow.smem_barriers = offsets.smem_barriers;
         base.flow.smem_bytes = offsets.smem_bytes;
-        base.wait_budget = S->cparams.copy_budget;
         cuda_check(adjoint_kernel_limits(static_cast<int>(limit), S->G > 8), "adjoint kernel limits");
         cuda_check(tape_kernel_limits(static_cast<int>(limit), S->G > 8), "taping kernel limits");
         cuda_check(cudaStreamSynchronize(S->stream), "rollout setup");
@@ -483,6 +482,7 @@ struct RolloutImpl {
         ap.damping = static_cast<float>(std::exp(-settings.velocity_damping * dt));
         ap.gravity = make_float3(settings.gravity.x, settings.gravity.y, settings.gravity.z);
         ap.iterations = settings.constraint_iterations;
+        ap.wait = S->cparams.wait;
         ap.ground = S->cparams.ground;
         ap.ground_normal = S->cparams.ground_normal;
         cudaLaunchAttribute attr[1];

@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_adjoint_kernel_t(con
     namespace cg = cooperative_groups;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ PilotAdjoint pa;
-    __shared__ int flow_dead;
+    __shared__ FlowLimit flow_limit;
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t me = cluster.block_rank();
     const ClusterInstance& I = *p.inst;
@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_adjoint_kernel_t(con
     const AdjointPilot* ap = p.tape.pilot;
 
     Flow flow;
-    flow_setup(flow, p.flow, me, smem, x_base, 0u, &flow_dead, I.status, p.wait_budget);
+    flow_setup(flow, p.flow, me, smem, x_base, 0u, &flow_limit, I.status, p.wait);
     const int S0 = I.kind[0].stages, S1 = I.kind[1].stages, S = S0 + S1;
     // this CTA's stage descriptors
     const uint4* desc = p.flow.stages + static_cast<size_t>(me) * S;
@@ -531,8 +531,8 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_adjoint_kernel_t(con
             stage_sync(1, blockDim.x);
         }
         if (tid == armer) {
-            if (barrier) flow_arm(flow.bar_base + barrier * 8u, flow.bytes[barrier]);
-            if (g == home_stage && phase > 0 && flow.home) flow_arm(flow.bar_base, flow.bytes[0]);
+            if (barrier) flow_arm_again(flow, barrier);
+            if (g == home_stage && phase > 0 && flow.home) flow_arm_again(flow, 0);
         }
     };
     for (; it >= 0; --it, ++phase) {
@@ -566,6 +566,7 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_adjoint_kernel_t(con
             __syncthreads();
         }
         if (p.flow.direct && (p.ground || I.susp_cta >= 0)) cluster.sync();
+        if (flow_ran_out(flow, phase)) continue;
         flow_send_out(flow, p.flow, xb);
         int g = S - 1;
         for (; g >= S0; --g) stage.template operator()<1>(g);
@@ -627,6 +628,7 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_adjoint_kernel_t(con
         p.g_mass[0] += pa.mass;
     }
     if (I.susp_cta < 0 && me == 0 && tid < 13) p.pb_in[tid] = 0.0f;
+    if (tid == 0) flow_drain(flow);
     cluster.sync();  // no CTA leaves while a peer may still read its memory
 }
 

@@ -13,6 +13,14 @@
 // count may run ahead of its arming); the phase cannot end before the
 // arming, which is its only arrival.  A node is not overwritten before its
 // reader is done: its next value exists only after the reader's result.
+//
+// A wait has a limit.  A CTA in which one has run out goes on to the end of
+// the step, so that every barrier of the block and of the cluster is met, but
+// it arms none of its own again (the phase that did not end has had its
+// arrival), and from the next iteration on it leaves out the stages and sends
+// nothing, so that the CTAs that wait for it run out in turn.  Before it
+// leaves it lets what is under way to it arrive (flow_drain).  The status word
+// makes the host drop the trial state.
 #pragma once
 
 #include "cluster_params.h"
@@ -21,15 +29,26 @@
 namespace swb {
 namespace dev {
 
+constexpr long long kFlowDrain = 200000;     // cycles, about 0.1 ms
+
+// The CTA's waits, in shared memory: what one that runs out works on.
+struct FlowLimit {
+    long long budget;      // cycles a wait may take
+    int* status;
+    uint32_t* bytes;       // Flow::bytes, set to 0 when a wait has run out
+    uint32_t barriers;
+    int ran_out;           // first iteration with a wait that ran out (one for the nodes that come
+                           // home counts to the next), kFlowNever, or -1: FlowWait::held
+};
+constexpr int kFlowNever = 0x7fffffff;
+
 struct Flow {
     uint32_t x_base;       // shared address of the node array
     uint32_t bar_base;     // shared address of the barriers
     uint32_t rank_base;    // the structure's first rank in the cluster
     const uint32_t* bytes; // per barrier (shared memory); [0]: the nodes that come home
     uint32_t out_lo, out_hi;
-    int* dead;             // shared: a wait of this CTA ran out
-    int* status;
-    long long budget;
+    FlowLimit* limit;
     bool home;             // nodes come home to this CTA from others
 };
 
@@ -49,12 +68,18 @@ __device__ __forceinline__ void stage_sync(uint32_t id, uint32_t threads) {
 __device__ __forceinline__ void flow_arm(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+// Arms this CTA's barrier `index` for the next iteration (one thread, behind a
+// barrier that follows every wait for this one), unless a wait has run out.
+__device__ __forceinline__ void flow_arm_again(const Flow& f, uint32_t index) {
+    const uint32_t bytes = f.bytes[index];
+    if (bytes) flow_arm(f.bar_base + index * 8u, bytes);
+}
 
 // This CTA's barriers (every thread; a cluster barrier must follow before
 // the first send).
 __device__ __forceinline__ void flow_setup(Flow& f, const ClusterFlowDev& F, uint32_t me, unsigned char* smem,
-                                           uint32_t x_base, uint32_t rank_base, int* dead, int* status,
-                                           long long budget) {
+                                           uint32_t x_base, uint32_t rank_base, FlowLimit* limit, int* status,
+                                           const FlowWait& wait) {
     uint32_t* bytes = reinterpret_cast<uint32_t*>(smem + F.smem_bytes);
     f.x_base = x_base;
     f.bar_base = smem_addr(smem + F.smem_barriers);
@@ -62,13 +87,13 @@ __device__ __forceinline__ void flow_setup(Flow& f, const ClusterFlowDev& F, uin
     f.bytes = bytes;
     f.out_lo = __ldg(F.out_begin + me);
     f.out_hi = __ldg(F.out_begin + me + 1);
-    f.dead = dead;
-    f.status = status;
-    f.budget = budget;
+    f.limit = limit;
     f.home = false;
-    if (threadIdx.x == 0) *dead = 0;
+    const uint32_t lo = __ldg(F.bytes_begin + me), n = F.direct ? 0u : __ldg(F.bytes_begin + me + 1) - lo;
+    // (direct schedules have no waits to run out)
+    const bool held = static_cast<int>(me) == wait.held && !F.direct;
+    if (threadIdx.x == 0) *limit = FlowLimit{wait.budget, status, bytes, n, held ? -1 : kFlowNever};
     if (F.direct) return;
-    const uint32_t lo = __ldg(F.bytes_begin + me), n = __ldg(F.bytes_begin + me + 1) - lo;
     for (uint32_t b = threadIdx.x; b < n; b += blockDim.x) {
         const uint32_t v = __ldg(F.bytes + lo + b);
         bytes[b] = v;
@@ -91,15 +116,16 @@ __device__ __forceinline__ bool flow_test(uint32_t bar, uint32_t parity) {
     return done != 0;
 }
 
-// (by value: a reference would put the caller's Flow into local memory)
-__device__ __noinline__ void flow_wait_slow(uint32_t bar, uint32_t parity, int* dead, int* status, long long budget) {
-    const long long start = clock64();
-    while (!flow_test(bar, parity)) {
-        if (*static_cast<volatile int*>(dead)) return;
-        if (clock64() - start > budget) {
-            // later waits of this CTA return at once, so the step ends
-            *static_cast<volatile int*>(dead) = 1;
-            atomicOr(status, kStatusSyncTimeout);
+__device__ __noinline__ void flow_wait_slow(uint32_t bar, uint32_t index, uint32_t iteration, FlowLimit* limit) {
+    volatile FlowLimit& l = *limit;
+    const long long start = clock64(), budget = l.budget;
+    while (!flow_test(bar, iteration & 1u)) {
+        if (l.ran_out != kFlowNever) return;
+        // (a structure with a wait that has run out in another CTA waits no longer)
+        if (clock64() - start > budget || (ld_relaxed_status(l.status) & kStatusFlowTimeout)) {
+            for (uint32_t b = 0; b < l.barriers; ++b) *static_cast<volatile uint32_t*>(l.bytes + b) = 0;
+            atomicMin(&limit->ran_out, static_cast<int>(iteration + (index == 0 ? 1u : 0u)));
+            atomicOr(l.status, kStatusFlowTimeout);
             return;
         }
     }
@@ -108,7 +134,22 @@ __device__ __noinline__ void flow_wait_slow(uint32_t bar, uint32_t parity, int* 
 // Waits for phase `iteration` of this CTA's barrier `index`.
 __device__ __forceinline__ void flow_wait(const Flow& f, uint32_t index, uint32_t iteration) {
     const uint32_t bar = f.bar_base + index * 8u;
-    if (!flow_test(bar, iteration & 1u)) flow_wait_slow(bar, iteration & 1u, f.dead, f.status, f.budget);
+    if (!flow_test(bar, iteration & 1u)) flow_wait_slow(bar, index, iteration, f.limit);
+}
+
+// Before iteration `iteration`: a wait of the ones before ran out (those for
+// the nodes of the last home-coming apart).  The same for every thread: all
+// that could answer otherwise lies behind a barrier of the block.
+__device__ __forceinline__ bool flow_ran_out(const Flow& f, uint32_t iteration) {
+    return static_cast<volatile FlowLimit*>(f.limit)->ran_out < static_cast<int>(iteration);
+}
+
+// Before this CTA leaves (one thread, behind a cluster barrier that follows
+// the iterations): where a wait has run out, nodes sent here may still be under
+// way.  They take a microsecond or two.
+__device__ __forceinline__ void flow_drain(const Flow& f) {
+    if (static_cast<volatile FlowLimit*>(f.limit)->ran_out == kFlowNever) return;
+    for (const long long start = clock64(); clock64() - start < kFlowDrain;) __nanosleep(1000);
 }
 
 // Sends a node where its word says (cluster_schedule.h, send_word).

@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_kernel_t(const __gri
     __shared__ DevPayloadDef pdef;  // suspension CTA: the payload definition, read on every line iteration
     __shared__ float3 shift_s;
     __shared__ uint32_t pbeg_s[kClusterMaxCtasDev + 1];  // the structure's patch starts
-    __shared__ int flow_dead;
+    __shared__ FlowLimit flow_limit;
     __shared__ double mom_scratch[kMaxWarps * kMomentumFields];
     __shared__ double mom_pred[kMomentumFields], mom_cur[kMomentumFields];
     __shared__ double mom_ptot[kMomentumFields], mom_tot[kMomentumFields];
@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_kernel_t(const __gri
     const int sctas = kPacked ? slot.ctas : p.ctas;
 
     Flow flow;
-    flow_setup(flow, I.flow, me, smem, x_base, rank_base, &flow_dead, I.status, p.copy_budget);
+    flow_setup(flow, I.flow, me, smem, x_base, rank_base, &flow_limit, I.status, p.wait);
     if (tid == 0) {
         mbar_init(&bar, 1);
         mbar_expect_tx(&bar, n * 16u);
@@ -736,8 +736,8 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_kernel_t(const __gri
             stage_sync(1, width);
         }
         if (tid == armer) {
-            if (barrier) flow_arm(flow.bar_base + barrier * 8u, flow.bytes[barrier]);
-            if (g == home_stage && it > 0 && flow.home) flow_arm(flow.bar_base, flow.bytes[0]);
+            if (barrier) flow_arm_again(flow, barrier);
+            if (g == home_stage && it > 0 && flow.home) flow_arm_again(flow, 0);
         }
     };
     // load-path cable sweeps (soft_body.cpp:1288-1317): a quarter of the
@@ -753,7 +753,8 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_kernel_t(const __gri
             if (n_pairs > 0) cluster.sync();  // every node is at home
             for (int q = 0; q < n_pairs; ++q) run_cable_pair(I, me, rank_base, x_base, lam0, first0, p.inv_dt2);
         }
-        flow_send_out(flow, I.flow, x);
+        const bool sweep = !flow_ran_out(flow, static_cast<uint32_t>(it));
+        if (sweep) flow_send_out(flow, I.flow, x);
         float4 *tape0 = nullptr, *tape1 = nullptr;
         uint32_t r0 = 0, r1 = 0;
         if constexpr (kTape) {
@@ -763,10 +764,12 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_kernel_t(const __gri
             tape1 = p.tape.dih + static_cast<size_t>(it) * 4 * r1;
         }
         int g = 0;
-        for (; g < S0; ++g) stage.template operator()<0>(g, lam0, first0, 0u, tape0, r0);
-        if constexpr (kMembrane)
-            for (; g < S0 + S2; ++g) stage.template operator()<2>(g, lam2, kind2 + first2, kind2, nullptr, 0u);
-        for (; g < S; ++g) stage.template operator()<1>(g, lam1, kind1 + first1, kind1, tape1, r1);
+        if (sweep) {
+            for (; g < S0; ++g) stage.template operator()<0>(g, lam0, first0, 0u, tape0, r0);
+            if constexpr (kMembrane)
+                for (; g < S0 + S2; ++g) stage.template operator()<2>(g, lam2, kind2 + first2, kind2, nullptr, 0u);
+            for (; g < S; ++g) stage.template operator()<1>(g, lam1, kind1 + first1, kind1, tape1, r1);
+        }
         for (; g < stages_c; ++g) cluster.sync();  // packed: the cluster's longer iterations
         if (susp && line_stage < 0 && owner) {
             __syncthreads();
@@ -777,7 +780,7 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_kernel_t(const __gri
             __syncthreads();
         }
         // this CTA's nodes are home
-        if (flow.home) flow_wait(flow, 0, static_cast<uint32_t>(it));
+        if (sweep && flow.home) flow_wait(flow, 0, static_cast<uint32_t>(it));
         if constexpr (kContact) contact_iteration(cctx, cluster);
         if (lines) {
             float4* line_tape = nullptr;
@@ -972,6 +975,7 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_kernel_t(const __gri
         I.origin_out[1] = I.origin_in[1] + static_cast<double>(shift.y);
         I.origin_out[2] = I.origin_in[2] + static_cast<double>(shift.z);
     }
+    if (tid == 0) flow_drain(flow);
     cluster.sync();  // no CTA leaves while a peer may still read its memory
 }
 

@@ -9,6 +9,15 @@
 
 namespace swb {
 
+// Waits for handed-over nodes: the cycles one may take (about 2 s), and, for
+// tests of a wait that runs out, the CTA of the structure that leaves its sweep
+// out (-1: none).
+constexpr long long kFlowWaitCycles = 4000000000LL;
+struct FlowWait {
+    long long budget = kFlowWaitCycles;
+    int held = -1;
+};
+
 namespace dev {
 constexpr int kClusterMaxThreads = 768;  // threads per CTA of the cluster step kernels at most
 constexpr int kClusterThreads = 512;     // ... as chosen: 128 registers a thread
@@ -326,6 +335,7 @@ struct ClusterParams {
     int iterations;
     int cable_pairs;               // load-path cable sweep pairs per substep (single-structure launches)
     long long copy_budget;
+    FlowWait wait;
     TapeStep tape;                 // taping launches: where this step's tape goes
     // contact launches: clusters after the first that join only the contact
     // detection phases (broadphase and swept queries), synchronised with the
@@ -367,7 +377,7 @@ struct AdjointParams {
     int iterations;
     uint32_t smem_vb, smem_lam0, smem_lam1, smem_acc0r, smem_acc0c, smem_acc1c;
     ClusterFlowDev flow;           // the reverse sweep's hand-overs
-    long long wait_budget;         // cycles a wait for nodes may take
+    FlowWait wait;
     int ground;                    // the frictionless ground plane of the forward step (ClusterParams)
     float3 ground_normal;
 };

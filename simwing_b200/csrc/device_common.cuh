@@ -18,6 +18,7 @@ enum : int {
     kStatusCopyTimeout = 8,
     kStatusMembrane = 16,
     kStatusContact = 32,   // status[1]: a kContact* detail code
+    kStatusFlowTimeout = 64,  // a wait for nodes from another CTA ran out (cluster_flow.cuh)
 };
 
 // Suspension detail codes, each one (phase, entity) of the reference's

@@ -666,7 +666,7 @@ void StructureImpl::setup_contact(const swb_solver_options& opt) {
 
 void StructureImpl::upload_cluster_tables() {
     ClusterParams& cp = cparams;
-    std::memset(&cp, 0, sizeof(cp));
+    cp = ClusterParams{};
     cp.ctas = G;
     const ClusterLayout layout = layout_of(csched);
     ClusterInstance base{};
@@ -1253,6 +1253,10 @@ swb_status decode_status(const int status[2], std::string& message) {
         message = "device-wide barrier timed out";
         return SWB_SYNC_TIMEOUT;
     }
+    if (status[0] & dev::kStatusFlowTimeout) {
+        message = "a wait for nodes handed over between the CTAs of a cluster timed out";
+        return SWB_SYNC_TIMEOUT;
+    }
     if (status[0] & dev::kStatusCopyTimeout) {
         message = "shared-memory staging timed out";
         return SWB_SYNC_TIMEOUT;
@@ -1790,6 +1794,18 @@ swb_status swb_structure_set_line_contact(swb_structure* s, const swb_line_conta
         cuda_check(cudaMemcpyAsync(m.d_lines, &L, sizeof(L), cudaMemcpyHostToDevice, m.stream), "line contact");
         m.line_contact = true;
         m.upload_instances();
+    });
+}
+
+swb_status swb_structure_set_wait_limit(swb_structure* s, int64_t cycles, int32_t held_cta) {
+    return guarded([&] {
+        if (!s) raise(SWB_INVALID_ARGUMENT, "null structure");
+        StructureImpl& m = s->s;
+        if (cycles < 0) raise(SWB_INVALID_ARGUMENT, "the wait limit must not be negative");
+        if (held_cta < -1 || (held_cta >= 0 && (!m.cluster_mode || held_cta >= m.G)))
+            raise(SWB_INVALID_ARGUMENT, "the held CTA is not one of the structure's cluster");
+        m.cparams.wait.budget = cycles > 0 ? cycles : kFlowWaitCycles;
+        m.cparams.wait.held = held_cta;
     });
 }
 
