@@ -24,6 +24,7 @@
 #include "cluster_params.h"
 #include "contact_phase.cuh"
 #include "device_common.cuh"
+#include "step_kernel.cuh"
 
 namespace swb {
 namespace dev {
@@ -32,31 +33,36 @@ struct SegmentClosest {
     float s, t;
 };
 
+// The arithmetic states its multiply-adds (step_kernel.cuh): which candidates
+// are projected is decided by one copy of it and the projection made by
+// another, on gathered nodes or in place, and all must round alike.
+
 // Parameters of the closest points p1 + s d1 and p2 + t d2 of two segments.
 __device__ __forceinline__ SegmentClosest segment_closest(float3 p1, float3 d1, float3 p2, float3 d2) {
     constexpr float eps = 1.0e-12f;
-    const float3 r = p1 - p2;
-    const float a = dot(d1, d1), e = dot(d2, d2), f = dot(d2, r);
+    const float3 r = rn_sub(p1, p2);
+    const float a = fma_dot(d1, d1), e = fma_dot(d2, d2), f = fma_dot(d2, r);
     SegmentClosest out{0.0f, 0.0f};
     if (a <= eps && e <= eps) return out;
     if (a <= eps) {
         out.t = fminf(fmaxf(f / e, 0.0f), 1.0f);
         return out;
     }
-    const float c = dot(d1, r);
+    const float c = fma_dot(d1, r);
     if (e <= eps) {
         out.s = fminf(fmaxf(-c / a, 0.0f), 1.0f);
         return out;
     }
-    const float b = dot(d1, d2), denom = a * e - b * b;
-    float s = denom != 0.0f ? fminf(fmaxf((b * f - c * e) / denom, 0.0f), 1.0f) : 0.0f;
-    float t = (b * s + f) / e;
+    const float b = fma_dot(d1, d2), denom = __fmaf_rn(a, e, -__fmul_rn(b, b));
+    const float over = __fmaf_rn(b, f, -__fmul_rn(c, e));
+    float s = denom != 0.0f ? fminf(fmaxf(over / denom, 0.0f), 1.0f) : 0.0f;
+    float t = __fmaf_rn(b, s, f) / e;
     if (t < 0.0f) {
         t = 0.0f;
         s = fminf(fmaxf(-c / a, 0.0f), 1.0f);
     } else if (t > 1.0f) {
         t = 1.0f;
-        s = fminf(fmaxf((b - c) / a, 0.0f), 1.0f);
+        s = fminf(fmaxf(__fadd_rn(b, -c) / a, 0.0f), 1.0f);
     }
     out.s = s;
     out.t = t;
@@ -226,25 +232,53 @@ __device__ void line_sort(const LineContactDev& L, uint32_t* scratch) {
     __syncthreads();
 }
 
+// The closest points of the segments A B and C D: where, and how far apart.
+struct LineGap {
+    SegmentClosest q;
+    float3 diff;
+    float dist;
+    // too near, and a direction to push along
+    __device__ __forceinline__ bool within(float gap) const { return dist < gap && dist > 0.0f; }
+};
+__device__ __forceinline__ LineGap line_gap(const float4& A, const float4& B, const float4& C, const float4& D) {
+    LineGap g;
+    const float3 a = f3(A), c = f3(C), d1 = rn_sub(f3(B), a), d2 = rn_sub(f3(D), c);
+    g.q = segment_closest(a, d1, c, d2);
+    float4 p = A, r = C;
+    fma_add(p, g.q.s, d1);
+    fma_add(r, g.q.t, d2);
+    g.diff = rn_sub(f3(p), f3(r));
+    g.dist = sqrtf(fma_dot(g.diff, g.diff));
+    return g;
+}
+
+// The nodes' shares of a correction, and the pair's effective inverse mass.
+struct LineWeights {
+    float a, b, c, d, sum;
+};
+__device__ __forceinline__ LineWeights line_weights(const float4& A, const float4& B, const float4& C, const float4& D,
+                                                    SegmentClosest q) {
+    const float rs = __fadd_rn(1.0f, -q.s), rt = __fadd_rn(1.0f, -q.t);
+    LineWeights w{__fmul_rn(A.w, rs), __fmul_rn(B.w, q.s), __fmul_rn(C.w, rt), __fmul_rn(D.w, q.t), 0.0f};
+    w.sum = __fmaf_rn(w.d, q.t, __fmaf_rn(w.c, rt, __fmaf_rn(w.a, rs, __fmul_rn(w.b, q.s))));
+    return w;
+}
+
 // One candidate's projection on its four end nodes: the closest points of
 // its two segments pushed apart to 2 x radius, rigidly, the correction shared
 // by inverse mass and barycentric weight.  False when they are apart (or
 // nothing can move): the nodes stay.
 __device__ __forceinline__ bool line_push(float4& A, float4& B, float4& Cn, float4& D, float gap) {
-    const float3 d1 = f3(B) - f3(A), d2 = f3(D) - f3(Cn);
-    const SegmentClosest q = segment_closest(f3(A), d1, f3(Cn), d2);
-    const float3 diff = (f3(A) + d1 * q.s) - (f3(Cn) + d2 * q.t);
-    const float dist = length(diff);
-    if (!(dist < gap) || !(dist > 0.0f)) return false;
-    const float3 nrm = diff / dist;
-    const float wa = A.w * (1.0f - q.s), wb = B.w * q.s, wc = Cn.w * (1.0f - q.t), wd = D.w * q.t;
-    const float W = wa * (1.0f - q.s) + wb * q.s + wc * (1.0f - q.t) + wd * q.t;
-    if (!(W > 0.0f)) return false;
-    const float dl = (gap - dist) / W;
-    A.x += nrm.x * wa * dl; A.y += nrm.y * wa * dl; A.z += nrm.z * wa * dl;
-    B.x += nrm.x * wb * dl; B.y += nrm.y * wb * dl; B.z += nrm.z * wb * dl;
-    Cn.x -= nrm.x * wc * dl; Cn.y -= nrm.y * wc * dl; Cn.z -= nrm.z * wc * dl;
-    D.x -= nrm.x * wd * dl; D.y -= nrm.y * wd * dl; D.z -= nrm.z * wd * dl;
+    const LineGap g = line_gap(A, B, Cn, D);
+    if (!g.within(gap)) return false;
+    const LineWeights w = line_weights(A, B, Cn, D, g.q);
+    if (!(w.sum > 0.0f)) return false;
+    const float3 nrm = g.diff / g.dist;
+    const float dl = __fadd_rn(gap, -g.dist) / w.sum;
+    fma_add(A, dl, rn_scale(nrm, w.a));
+    fma_add(B, dl, rn_scale(nrm, w.b));
+    fma_add(Cn, -dl, rn_scale(nrm, w.c));
+    fma_add(D, -dl, rn_scale(nrm, w.d));
     return true;
 }
 
@@ -287,8 +321,7 @@ __device__ __noinline__ void line_project_near(const LineContactDev& L, Addr add
     }
     __syncthreads();
     const uint32_t n = min(L.count[0], L.capacity), lane = threadIdx.x & 31u;
-    // a hair wider than the projection's own test
-    const float gap = 2.0f * L.radius, wide = gap * 1.0001f;
+    const float gap = 2.0f * L.radius;
     bool any = false;
     for (uint32_t k0 = threadIdx.x & ~31u; k0 < n; k0 += blockDim.x) {
         bool hit = false;
@@ -296,9 +329,7 @@ __device__ __noinline__ void line_project_near(const LineContactDev& L, Addr add
             const uint2 c = L.cand_near[k0 + lane];
             const float4 A = ld_own(y + 16u * (c.x & 0xffffu)), B = ld_own(y + 16u * (c.x >> 16)),
                          Cn = ld_own(y + 16u * (c.y & 0xffffu)), D = ld_own(y + 16u * (c.y >> 16));
-            const float3 d1 = f3(B) - f3(A), d2 = f3(D) - f3(Cn);
-            const SegmentClosest q = segment_closest(f3(A), d1, f3(Cn), d2);
-            hit = !(length((f3(A) + d1 * q.s) - (f3(Cn) + d2 * q.t)) > wide);
+            hit = line_gap(A, B, Cn, D).within(gap);
         }
         const uint32_t word = __ballot_sync(0xffffffffu, hit);
         if (lane == 0) start[k0 >> 5] = word;
@@ -419,17 +450,10 @@ __device__ __forceinline__ double dot(LV3 a, LV3 b) { return a.x * b.x + a.y * b
 // (s free) and d2 . (P - Q) = 0 (t free), and their adjoints pass through
 // those conditions (implicit function).
 __device__ __forceinline__ void line_reverse_one(const float4 in[4], float gap_f, float3 g3[4]) {
-    const SegmentClosest q = segment_closest(f3(in[0]), f3(in[1]) - f3(in[0]), f3(in[2]), f3(in[3]) - f3(in[2]));
-    {
-        // the forward's own test, in its own arithmetic
-        const float3 d1 = f3(in[1]) - f3(in[0]), d2 = f3(in[3]) - f3(in[2]);
-        const float3 df = (f3(in[0]) + d1 * q.s) - (f3(in[2]) + d2 * q.t);
-        const float dist = length(df);
-        if (!(dist < gap_f) || !(dist > 0.0f)) return;
-        const float Wf = in[0].w * (1.0f - q.s) * (1.0f - q.s) + in[1].w * q.s * q.s +
-                         in[2].w * (1.0f - q.t) * (1.0f - q.t) + in[3].w * q.t * q.t;
-        if (!(Wf > 0.0f)) return;
-    }
+    // the forward's own tests, in its own arithmetic
+    const LineGap near = line_gap(in[0], in[1], in[2], in[3]);
+    if (!near.within(gap_f) || !(line_weights(in[0], in[1], in[2], in[3], near.q).sum > 0.0f)) return;
+    const SegmentClosest q = near.q;
     const double gap = gap_f, s = q.s, t = q.t;
     const LV3 A = lv3(in[0]), B = lv3(in[1]), C = lv3(in[2]), D = lv3(in[3]);
     LV3 g[4] = {lv3(g3[0]), lv3(g3[1]), lv3(g3[2]), lv3(g3[3])};
