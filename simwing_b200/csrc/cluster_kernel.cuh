@@ -520,6 +520,7 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_kernel_t(const __gri
         cctx.grid.blocks = gridDim.x;
         cctx.order = smem_addr(smem + I.smem_order);
         cctx.order_bytes = I.order_bytes;
+        cctx.sink = smem_addr(mom_scratch);  // (no momentum guard beside contact)
         // multipliers and records restart every substep (beginContactSubstep,
         // contact.cpp:1043-1055)
         if (me == 0 && tid == 0) {

@@ -199,6 +199,27 @@ struct ClusterLayout {
 };
 ClusterLayout layout_of(const ClusterSchedule& s);
 
+// Shared memory of a contact launch with the key-ordered passes' links (11
+// bytes a candidate in contact, contact_phase.cuh).  Shared memory comes off
+// the L1 cache in steps, and the detection phases read through that cache
+// (with 192 KB of links the row passes of 24 x 24 sheets take 2.0 ms a step
+// against 1.1 ms), but links that do not fit cost more still (40 x 40 sheets:
+// 22 ms of rounds against 13 ms).  So: the smallest step that holds one
+// candidate in contact per candidate row, about what a landed sheet has (24 x
+// 24 sheets: 4,500 rows, 3,900 in contact), and the first step when none does.
+constexpr uint32_t kContactSharedSteps[] = {124 * 1024, 156 * 1024, 188 * 1024, 218 * 1024};
+constexpr uint32_t kContactLinkBytes = 11;
+// Their bytes behind a layout of `layout` bytes in a launch that may take `cap`;
+// 0 where it leaves none (the links stay in global memory).
+inline uint32_t contact_link_bytes(uint32_t layout, uint64_t rows, uint64_t cap) {
+    const uint64_t want = layout + rows * kContactLinkBytes + 256;
+    uint64_t limit = kContactSharedSteps[0];
+    for (uint32_t step : kContactSharedSteps)
+        if (limit < want && step >= want) limit = step;
+    limit = limit < cap ? limit : cap;
+    return limit > layout ? static_cast<uint32_t>(limit - layout) & ~15u : 0u;
+}
+
 // Stages a line iteration may run beside: one takes about 5 us, a stage of a
 // wing 0.5 to 1 us.
 constexpr int kLineWindow = 8;

@@ -97,6 +97,7 @@ struct ContactCtx {
     GridBarrier grid;
     uint32_t order;            // shared memory of the key-ordered passes (run_order): address
     uint32_t order_bytes;
+    uint32_t sink;             // 16 bytes of shared memory nobody reads, for fetch_line's copies
 };
 
 // The barrier between two detection phases.
@@ -700,7 +701,6 @@ __device__ __forceinline__ uint32_t atom_shared_add(uint32_t addr, uint32_t v) {
 // The links of run_order in shared memory: per item its followers (0xffff:
 // none), the count of items it still waits for, a place in the queue.
 constexpr uint32_t kOrderItemBytes = 11;
-constexpr uint32_t kOrderSink = 32;  // bytes before them: where fetch_line's copies go
 // Runs work(item) for `items` items in an order that keeps, for every node,
 // the items touching it in item order (the calling block, after
 // cluster_order): rounds, each running together the items whose earlier
@@ -727,9 +727,9 @@ template <class Work, class Ahead>
 __device__ __forceinline__ void run_order(const ContactCtx& c, uint32_t items, Work work, Ahead ahead) {
     const ContactDev& C = *c.C;
     __shared__ uint32_t round_n[3];  // items of this round, of the next one, the count being cleared
-    const bool shared = items < 0xffffu && kOrderSink + (items + 8) * kOrderItemBytes <= c.order_bytes;
-    const uint32_t sink = c.order;
-    const uint32_t succ = c.order + kOrderSink, near_queue = succ + 8 * items,
+    const bool shared = items < 0xffffu && (items + 8) * kOrderItemBytes <= c.order_bytes;
+    const uint32_t sink = c.sink;
+    const uint32_t succ = c.order, near_queue = succ + 8 * items,
                    near_waits = (near_queue + 2 * items + 3) & ~3u;  // a byte per item
     if (threadIdx.x < 3) round_n[threadIdx.x] = 0;
     if (shared)

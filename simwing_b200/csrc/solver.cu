@@ -710,14 +710,8 @@ void StructureImpl::upload_cluster_tables() {
     if (def.has_contact) {
         // the links of the key-ordered contact passes, beside the patch
         base.smem_order = layout.total;
-        const size_t rows = contact_surface.vertices.size() + contact_surface.edges.size();
-        const size_t want = layout.total + rows * kContactLinkBytes + 256;
-        size_t limit = kContactSharedSteps[0];
-        for (size_t step : kContactSharedSteps)
-            if (limit < want && step >= want) limit = step;
-        limit = std::min(limit, smem_cap);
         base.order_bytes =
-            static_cast<uint32_t>(std::max<size_t>(limit > layout.total ? (limit - layout.total) & ~size_t{15} : 0, 32));
+            contact_link_bytes(layout.total, contact_surface.vertices.size() + contact_surface.edges.size(), smem_cap);
         cluster_smem += base.order_bytes;
     }
     base.seam_offsets = dupload(owned, csched.seam_offsets, stream);

@@ -59,17 +59,6 @@ constexpr int kMaxContactHelpers = 8;
 // their detection phases on the structure's cluster.
 constexpr uint32_t kContactHelperRows = 16384;
 
-// Shared memory of a contact launch with the key-ordered passes' links (11
-// bytes a candidate in contact, contact_phase.cuh).  Shared memory comes off
-// the L1 cache in steps, and the detection phases read through that cache
-// (with 192 KB of links the row passes of 24 x 24 sheets take 2.0 ms a step
-// against 1.1 ms), but links that do not fit cost more still (40 x 40 sheets:
-// 22 ms of rounds against 13 ms).  So: the smallest step that holds one
-// candidate in contact per candidate row, about what a landed sheet has (24 x
-// 24 sheets: 4,500 rows, 3,900 in contact), and the first step when none does.
-constexpr size_t kContactSharedSteps[] = {124 * 1024, 156 * 1024, 188 * 1024, 218 * 1024};
-constexpr size_t kContactLinkBytes = 11;
-
 // Diagnostics partial sums per block.
 constexpr int kDiagFields = 16;
 
