@@ -37,6 +37,7 @@ struct FlowLimit {
     int* status;
     uint32_t* bytes;       // Flow::bytes, set to 0 when a wait has run out
     uint32_t barriers;
+    uint32_t home;         // shared address of the barrier of the nodes that come home
     int ran_out;           // first iteration with a wait that ran out (one for the nodes that come
                            // home counts to the next), kFlowNever, or -1: FlowWait::held
 };
@@ -92,7 +93,7 @@ __device__ __forceinline__ void flow_setup(Flow& f, const ClusterFlowDev& F, uin
     const uint32_t lo = __ldg(F.bytes_begin + me), n = F.direct ? 0u : __ldg(F.bytes_begin + me + 1) - lo;
     // (direct schedules have no waits to run out)
     const bool held = static_cast<int>(me) == wait.held && !F.direct;
-    if (threadIdx.x == 0) *limit = FlowLimit{wait.budget, status, bytes, n, held ? -1 : kFlowNever};
+    if (threadIdx.x == 0) *limit = FlowLimit{wait.budget, status, bytes, n, f.bar_base, held ? -1 : kFlowNever};
     if (F.direct) return;
     for (uint32_t b = threadIdx.x; b < n; b += blockDim.x) {
         const uint32_t v = __ldg(F.bytes + lo + b);
@@ -116,15 +117,14 @@ __device__ __forceinline__ bool flow_test(uint32_t bar, uint32_t parity) {
     return done != 0;
 }
 
-__device__ __noinline__ void flow_wait_slow(uint32_t bar, uint32_t index, uint32_t iteration, FlowLimit* limit) {
+__device__ __noinline__ void flow_wait_slow(uint32_t bar, uint32_t iteration, FlowLimit* limit) {
     volatile FlowLimit& l = *limit;
     const long long start = clock64(), budget = l.budget;
-    while (!flow_test(bar, iteration & 1u)) {
-        if (l.ran_out != kFlowNever) return;
+    while (l.ran_out == kFlowNever && !flow_test(bar, iteration & 1u)) {
         // (a structure with a wait that has run out in another CTA waits no longer)
         if (clock64() - start > budget || (ld_relaxed_status(l.status) & kStatusFlowTimeout)) {
             for (uint32_t b = 0; b < l.barriers; ++b) *static_cast<volatile uint32_t*>(l.bytes + b) = 0;
-            atomicMin(&limit->ran_out, static_cast<int>(iteration + (index == 0 ? 1u : 0u)));
+            atomicMin(&limit->ran_out, static_cast<int>(iteration + (bar == l.home ? 1u : 0u)));
             atomicOr(l.status, kStatusFlowTimeout);
             return;
         }
@@ -134,7 +134,7 @@ __device__ __noinline__ void flow_wait_slow(uint32_t bar, uint32_t index, uint32
 // Waits for phase `iteration` of this CTA's barrier `index`.
 __device__ __forceinline__ void flow_wait(const Flow& f, uint32_t index, uint32_t iteration) {
     const uint32_t bar = f.bar_base + index * 8u;
-    if (!flow_test(bar, iteration & 1u)) flow_wait_slow(bar, index, iteration, f.limit);
+    if (!flow_test(bar, iteration & 1u)) flow_wait_slow(bar, iteration, f.limit);
 }
 
 // Before iteration `iteration`: a wait of the ones before ran out (those for

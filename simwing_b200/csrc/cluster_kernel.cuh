@@ -754,18 +754,17 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_kernel_t(const __gri
             if (n_pairs > 0) cluster.sync();  // every node is at home
             for (int q = 0; q < n_pairs; ++q) run_cable_pair(I, me, rank_base, x_base, lam0, first0, p.inv_dt2);
         }
-        const bool sweep = !flow_ran_out(flow, static_cast<uint32_t>(it));
-        if (sweep) flow_send_out(flow, I.flow, x);
-        float4 *tape0 = nullptr, *tape1 = nullptr;
-        uint32_t r0 = 0, r1 = 0;
-        if constexpr (kTape) {
-            r0 = p.tape.r0;
-            r1 = p.tape.r1;
-            tape0 = p.tape.dist + static_cast<size_t>(it) * 2 * r0;
-            tape1 = p.tape.dih + static_cast<size_t>(it) * 4 * r1;
-        }
         int g = 0;
-        if (sweep) {
+        if (!flow_ran_out(flow, static_cast<uint32_t>(it))) [[likely]] {
+            flow_send_out(flow, I.flow, x);
+            float4 *tape0 = nullptr, *tape1 = nullptr;
+            uint32_t r0 = 0, r1 = 0;
+            if constexpr (kTape) {
+                r0 = p.tape.r0;
+                r1 = p.tape.r1;
+                tape0 = p.tape.dist + static_cast<size_t>(it) * 2 * r0;
+                tape1 = p.tape.dih + static_cast<size_t>(it) * 4 * r1;
+            }
             for (; g < S0; ++g) stage.template operator()<0>(g, lam0, first0, 0u, tape0, r0);
             if constexpr (kMembrane)
                 for (; g < S0 + S2; ++g) stage.template operator()<2>(g, lam2, kind2 + first2, kind2, nullptr, 0u);
@@ -781,7 +780,7 @@ __global__ void __launch_bounds__(kMaxThreads) xpbd_cluster_kernel_t(const __gri
             __syncthreads();
         }
         // this CTA's nodes are home
-        if (sweep && flow.home) flow_wait(flow, 0, static_cast<uint32_t>(it));
+        if (flow.home) flow_wait(flow, 0, static_cast<uint32_t>(it));
         if constexpr (kContact) contact_iteration(cctx, cluster);
         if (lines) {
             float4* line_tape = nullptr;
