@@ -616,6 +616,24 @@ ClusterLayout layout_of(const ClusterSchedule& s) {
     return L;
 }
 
+LineWindow line_window(const ClusterSchedule& S, int threads) {
+    LineWindow w;
+    if (S.line_stage < 0) return w;
+    const int G = total_stages(S);
+    for (int g = G - 1; g >= S.line_stage; --g) {
+        int k, s;
+        global_stage(S, g, k, s);
+        const ClusterKind& K = S.kinds[k];
+        const size_t o = static_cast<size_t>(S.susp_cta) * (K.stages + 1) + s;
+        const uint32_t n = K.offsets[o + 1] - K.offsets[o];
+        if (static_cast<int64_t>(n) > threads - 32) break;
+        if (G - g >= 2) w.first = g;
+        w.records = std::max(w.records, n);
+    }
+    if (w.first < 0) w.records = 0;
+    return w;
+}
+
 bool build_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_t>& suspension_nodes, int ctas,
                             ClusterSchedule& S, bool split, size_t shared_limit) {
     S = ClusterSchedule{};
@@ -798,13 +816,7 @@ bool build_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_t
         while (first > 0 && Sg - first < kLineWindow && !stage_touches(d, S, attached, first - 1)) --first;
         if (Sg - first >= 2) {
             S.line_stage = first;
-            for (int g = first; g < Sg; ++g) {
-                int k, s;
-                global_stage(S, g, k, s);
-                const ClusterKind& K = S.kinds[k];
-                const size_t o = static_cast<size_t>(S.susp_cta) * (K.stages + 1) + s;
-                S.line_owner_records = std::max(S.line_owner_records, K.offsets[o + 1] - K.offsets[o]);
-            }
+            S.line_owner_records = line_window(S, std::numeric_limits<int>::max()).records;
         }
     }
 

@@ -224,6 +224,16 @@ inline uint32_t contact_link_bytes(uint32_t layout, uint64_t rows, uint64_t cap)
 // wing 0.5 to 1 us.
 constexpr int kLineWindow = 8;
 
+// The stages of the schedule's line iteration window that a block of `threads`
+// threads leaves a warp idle in (the suspension CTA's records fit the others),
+// from the last one back: the first of them, -1 when they are fewer than two,
+// and the suspension CTA's largest record count in them.
+struct LineWindow {
+    int first = -1;
+    uint32_t records = 0;
+};
+LineWindow line_window(const ClusterSchedule& s, int threads);
+
 // Returns false (and leaves `out` empty) when the mesh does not fit one
 // cluster of `ctas` CTAs (a patch over kClusterPatchNodes nodes).  The
 // forward flow is direct when its layout with ghosts would exceed

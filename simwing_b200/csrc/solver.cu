@@ -322,11 +322,15 @@ void StructureImpl::build(const swb_structure_definition& definition, const swb_
     if (threads % 32 != 0 || threads < 32 || threads > (cluster_mode ? dev::kClusterMaxThreads : 1024))
         raise(SWB_INVALID_ARGUMENT, "block_threads out of range for the chosen schedule");
     if (cluster_mode && csched.line_stage >= 0) {
-        // the line iteration needs a warp of the suspension CTA that is idle
-        // in its two stages
-        const int need = static_cast<int>((csched.line_owner_records + 31) / 32 * 32 + 32);
-        if (opt.block_threads <= 0 && need > threads && need <= dev::kClusterThreads) threads = need;
-        if (need > threads) csched.line_stage = -1;
+        // the line iteration needs a warp of the suspension CTA that is idle in
+        // its stages: in a block of the caller's, as many of them as leave one,
+        // else a block wide enough for as many as a block may be
+        const bool given = opt.block_threads > 0;
+        const LineWindow w = line_window(csched, given ? threads : std::max(threads, dev::kClusterThreads));
+        if (!given && w.first >= 0)
+            threads = std::max(threads, static_cast<int>((w.records + 31) / 32 * 32 + 32));
+        csched.line_stage = w.first;
+        csched.line_owner_records = w.records;
     }
     // the reverse sweep takes one record per thread
     reverse_threads = std::max(threads, static_cast<int>(std::clamp<uint32_t>((widest_single + 31) / 32 * 32, 64, 512)));

@@ -2,6 +2,10 @@
 all of them: riser endpoints that no constraint touches.  The window decides
 only when the line iteration runs, so a block too narrow to have one gives the
 same bits, forward and in a rollout's gradients."""
+import os
+import shutil
+import subprocess
+
 import numpy as np
 import pytest
 
@@ -42,6 +46,21 @@ def test_window_of_every_stage_is_planned(ctas):
     # a window: no barrier of the line iteration's own beside the stages
     assert 2 <= r.local_stages_per_iteration <= 8
     assert r.cluster_barriers_per_iteration == r.local_stages_per_iteration
+
+
+def test_window_of_a_block(tmp_path):
+    """tests/cpp/line_window_test.cpp: the window for every block width."""
+    cxx = shutil.which("g++")
+    if cxx is None:
+        pytest.skip("g++ not available")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    lib = os.path.join(root, "simwing_b200")
+    out = tmp_path / "line_window_test"
+    subprocess.run([cxx, "-std=c++20", "-O1", "-Wall", "-Wextra", "-Werror", "-I", os.path.join(root, "include"),
+                    os.path.join(root, "tests", "cpp", "line_window_test.cpp"), "-L", lib, "-lsimwing_b200",
+                    f"-Wl,-rpath,{lib}", "-o", str(out)], check=True)
+    r = subprocess.run([str(out)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout
 
 
 @pytest.mark.gpu
