@@ -109,31 +109,6 @@ struct RolloutImpl {
         cuda_check(cudaMemcpyAsync(to.origin, from.origin, 3 * sizeof(double), cudaMemcpyDeviceToDevice, st), "copy");
     }
 
-    // Shared memory of the reverse kernel with hand-overs `f`: the node
-    // adjoints (with ghosts unless direct) at 0, their start adjoints, the
-    // records' multiplier and parameter adjoints, the stage descriptors where
-    // they fit, the barriers.
-    uint32_t reverse_layout(const ClusterSchedule& cs, const ClusterFlow& f, size_t limit) {
-        const uint32_t m0 = cs.kinds[0].max_cta_records, m1 = cs.kinds[1].max_cta_records;
-        uint32_t off = al16((f.direct ? cs.max_patch : cs.max_local) * 16u);
-        base.smem_vb = off; off = al16(off + cs.max_patch * 16u);
-        base.smem_lam0 = off; off = al16(off + m0 * 4u);
-        base.smem_lam1 = off; off = al16(off + m1 * 4u);
-        base.smem_acc0r = off; off = al16(off + m0 * 4u);
-        base.smem_acc0c = off; off = al16(off + m0 * 4u);
-        base.smem_acc1c = off; off = al16(off + m1 * 4u);
-        base.flow.smem_barriers = off;
-        if (!f.direct) off = al16(off + f.max_barriers * 8u);
-        base.flow.smem_bytes = off;
-        if (!f.direct) off = al16(off + f.max_barriers * 4u);
-        base.flow.smem_stages = kStagesInGlobal;
-        if (total_stages(cs) <= kSharedStages && off + total_stages(cs) * 16u <= limit) {
-            base.flow.smem_stages = off;
-            off = al16(off + total_stages(cs) * 16u);
-        }
-        return smem = off;
-    }
-
     void build(StructureImpl& s, int n_steps, int every) {
         S = &s;
         if (!S->cluster_mode)
@@ -232,20 +207,23 @@ struct RolloutImpl {
         cudaDeviceProp prop{};
         cuda_check(cudaGetDeviceProperties(&prop, S->device), "cudaGetDeviceProperties");
         const size_t limit = dynamic_smem_limit(prop);
-        ClusterFlow reverse = build_flow(S->def, cs, true, cs.forward.direct);
-        if (reverse_layout(cs, reverse, limit) > limit && !reverse.direct) {
-            reverse = build_flow(S->def, cs, true, true);
-            reverse_layout(cs, reverse, limit);
-        }
+        const ClusterFlow reverse = build_reverse_flow(S->def, cs, limit);
         verify_flow(S->def, cs, reverse, true);
+        const ReverseLayout L = reverse_layout_of(cs, reverse, limit);
+        smem = L.total;
         if (smem > limit)
             raise(SWB_UNSUPPORTED, "the reverse sweep needs " + std::to_string(smem) +
                                        " B of shared memory per CTA; build the structure with more cluster CTAs");
-        const ClusterFlowDev offsets = base.flow;
+        base.smem_vb = L.start;
+        base.smem_lam0 = L.lambda[0];
+        base.smem_lam1 = L.lambda[1];
+        base.smem_acc0r = L.rest;
+        base.smem_acc0c = L.compliance[0];
+        base.smem_acc1c = L.compliance[1];
         base.flow = upload_flow(cs, reverse, owned, S->stream);
-        base.flow.smem_stages = offsets.smem_stages;
-        base.flow.smem_barriers = offsets.smem_barriers;
-        base.flow.smem_bytes = offsets.smem_bytes;
+        base.flow.smem_stages = L.stages;
+        base.flow.smem_barriers = L.barriers;
+        base.flow.smem_bytes = L.bytes;
         cuda_check(adjoint_kernel_limits(static_cast<int>(limit), S->G > 8), "adjoint kernel limits");
         cuda_check(tape_kernel_limits(static_cast<int>(limit), S->G > 8), "taping kernel limits");
         cuda_check(cudaStreamSynchronize(S->stream), "rollout setup");

@@ -859,6 +859,38 @@ bool build_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_t
     return true;
 }
 
+ReverseLayout reverse_layout_of(const ClusterSchedule& s, const ClusterFlow& f, size_t limit) {
+    auto align = [](uint64_t v) { return (v + 15) & ~uint64_t{15}; };
+    const uint64_t m[2] = {s.kinds[0].max_cta_records * 4ull, s.kinds[1].max_cta_records * 4ull};
+    ReverseLayout L;
+    uint64_t off = align((f.direct ? s.max_patch : s.max_local) * 16ull);
+    auto take = [&](uint64_t bytes) {
+        const uint64_t at = off;
+        off = align(off + bytes);
+        return static_cast<uint32_t>(at);
+    };
+    L.start = take(s.max_patch * 16ull);
+    L.lambda[0] = take(m[0]);
+    L.lambda[1] = take(m[1]);
+    L.rest = take(m[0]);
+    L.compliance[0] = take(m[0]);
+    L.compliance[1] = take(m[1]);
+    L.barriers = take(f.direct ? 0 : f.max_barriers * 8ull);
+    L.bytes = take(f.direct ? 0 : f.max_barriers * 4ull);
+    const int G = total_stages(s);
+    L.stages = G <= kSharedStages && off + G * 16ull <= limit ? take(G * 16ull) : kStagesInGlobal;
+    L.total = static_cast<uint32_t>(std::min<uint64_t>(off, 0xffffffffu));
+    return L;
+}
+
+ClusterFlow build_reverse_flow(const OwnedDefinition& d, const ClusterSchedule& s, size_t limit) {
+    if (!s.forward.direct) {
+        ClusterFlow f = build_flow(d, s, true, false);
+        if (f.max_barriers <= kSendBarriers && reverse_layout_of(s, f, limit).total <= limit) return f;
+    }
+    return build_flow(d, s, true, true);
+}
+
 // Checks a flow: walking the stages, every record finds each of its nodes in
 // its own CTA's array (or, in a direct schedule, marked with the node's
 // home), counted on the barrier its stage waits on; every node ends at home;

@@ -244,8 +244,24 @@ bool build_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_t
 // The hand-overs of one sweep direction (see ClusterFlow).
 ClusterFlow build_flow(const OwnedDefinition& d, const ClusterSchedule& s, bool reverse, bool direct);
 
+// Dynamic shared memory of the reverse kernel with hand-overs `f`, byte
+// offsets: the node adjoints (with ghosts unless direct) at 0, their start
+// adjoints, the records' multiplier and parameter adjoints (rest lengths of
+// distances, compliances), then as in ClusterLayout; the stage descriptors are
+// left in global memory where they would exceed `limit`.
+struct ReverseLayout {
+    uint32_t start = 0, lambda[2] = {0, 0}, rest = 0, compliance[2] = {0, 0};
+    uint32_t stages = 0, barriers = 0, bytes = 0, total = 0;
+};
+ReverseLayout reverse_layout_of(const ClusterSchedule& s, const ClusterFlow& f, size_t limit);
+
+// The reverse sweep's hand-overs: direct where the forward's are, where
+// handing over would exceed `limit` bytes of shared memory, or where a CTA has
+// more receiving stages than a send word can name.
+ClusterFlow build_reverse_flow(const OwnedDefinition& d, const ClusterSchedule& s, size_t limit);
+
 // Checks a flow of a schedule; raises on failure (verify_cluster_schedule
-// checks the forward one).
+// checks the forward one, a planned schedule's reverse ones are checked too).
 void verify_flow(const OwnedDefinition& d, const ClusterSchedule& s, const ClusterFlow& f, bool reverse);
 
 // Stage descriptors of a flow, [ctas * stages] (global stages): the first

@@ -754,8 +754,12 @@ swb_status plan(const swb_structure_definition* definition, const swb_solver_opt
                 const size_t bytes = cluster_shared_bytes(C);
                 // opt-in shared memory less the kernels' static shared memory
                 // (under 6 KB; the device build reads the exact figure)
-                if (bytes > 227 * 1024 - 6144) continue;
+                const size_t limit = 227 * 1024 - 6144;
+                if (bytes > limit) continue;
                 verify_cluster_schedule(def, susp, C);
+                // the reverse sweep of a rollout, as it would run and in place
+                verify_flow(def, C, build_reverse_flow(def, C, limit), true);
+                verify_flow(def, C, build_flow(def, C, true, true), true);
                 std::memset(out, 0, sizeof(*out));
                 out->blocks = C.ctas;
                 out->cluster_ctas = C.ctas;
