@@ -26,8 +26,6 @@
 namespace swb {
 namespace {
 
-uint32_t al16(uint32_t v) { return (v + 15u) & ~15u; }
-
 template <class T>
 T* ralloc(std::vector<void*>& owned, size_t count) {
     void* p = nullptr;

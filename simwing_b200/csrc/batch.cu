@@ -31,8 +31,6 @@
 namespace swb {
 namespace {
 
-uint32_t align16u(uint32_t v) { return (v + 15u) & ~15u; }
-
 template <class T>
 T* batch_alloc(std::vector<void*>& owned, size_t count) {
     void* p = nullptr;

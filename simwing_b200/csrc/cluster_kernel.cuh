@@ -12,8 +12,8 @@
 //
 // What bounds the sweep: a stage is one dependent chain (node loads, the
 // projection, node stores, the CTA barrier), 1,200 of them per step of the
-// full wing, with at most one record per thread.  The stage loop is
-// therefore kept short: records, send words and stage descriptors are
+// full wing, with at most one dihedral or membrane record, or two distance
+// records side by side, per thread.  The stage loop is therefore kept short: records, send words and stage descriptors are
 // fetched one stage ahead, references are local, and no cluster barrier or
 // fence stands between two stages.  With a cluster barrier after every stage
 // and foreign nodes read and written in place, the full wing (16 CTAs) took
@@ -50,12 +50,6 @@ __device__ __forceinline__ uint32_t node_addr(uint32_t ref, uint32_t me, uint32_
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank + rank_base));
     return remote;
 }
-
-// The two halves of a cluster barrier, for a warp that works between its
-// arrival and its wait (arrive releases, wait acquires; every lane of the
-// warp executes both).
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
 
 // ---- momentum guard of free structures (soft_body.cpp:119-190) -------------
 // Sums over a CTA's free nodes, in double: [0] mass, [1..3] sum m x,

@@ -148,15 +148,15 @@ struct ContactDev {
                                        // detail code (contact_fail_at); all ones when none failed
     // order links of a key-ordered pass (cluster_order, run_order): node
     // buckets of the (node, item) pairs, each item's followers through its
-    // nodes, the count of items each one still waits for, and the two
-    // rounds' item lists
+    // nodes, the count of items each one still waits for, and the rounds'
+    // items one after the other (where they are not in shared memory)
     uint32_t* lv_node_start;           // [slots + 1] counts, then bucket starts
     uint32_t* lv_node_fill;            // [slots]
     uint32_t* lv_pairs;                // [6 * cand_cap]
     uint32_t* lv_succ;                 // [6 * cand_cap]
     uint32_t* lv_nsucc;                // [cand_cap]
     uint32_t* lv_npred;                // [cand_cap]
-    uint32_t* lv_front;                // [2 * cand_cap]
+    uint32_t* lv_front;                // [cand_cap]
 };
 
 // Line-line contact of one structure: the cable segments (node references

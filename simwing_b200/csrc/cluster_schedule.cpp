@@ -693,9 +693,7 @@ bool build_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_t
             K.stages = dsatur_colour(nodes, counts, colour);
             K.stages = reduce_colours(nodes, counts, N, K.stages, colour, kColourSearchMoves);
             balance_colours(nodes, counts, cta_of, ctas, N, K.stages, colour);
-            K.cluster_sync.assign(K.stages, 1);
-            K.interior_stages = 0;
-            K.boundary_stages = K.stages;
+            K.sync_stages = K.stages;
         } else {
             // Split stages.  A record whose nodes all lie in its CTA's patch
             // is interior; the others (boundary records) are coloured first
@@ -704,9 +702,8 @@ bool build_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_t
             // take the smallest colour free at all of their nodes,
             // boundary colours included, and open a colour of their own
             // only where none is.  The stages of interior-only colours run
-            // first, each closed by a CTA barrier (a CTA touches its own
-            // patch only), the last by a cluster barrier; every stage with
-            // boundary records is closed by a cluster barrier.
+            // first (a CTA touches its own patch only), then the stages with
+            // boundary records.
             std::vector<size_t> ids;
             std::vector<std::array<uint32_t, 4>> sub;
             std::vector<int> subc;
@@ -765,10 +762,7 @@ bool build_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_t
             for (int c = 0; c < total; ++c) stage_of[c] = c >= B ? c - B : inner_only + c;
             for (size_t i = 0; i < m; ++i) colour[i] = stage_of[colour[i]];
             K.stages = total;
-            K.interior_stages = inner_only;
-            K.boundary_stages = B;
-            K.cluster_sync.assign(K.stages, 1);
-            for (int g = 0; g + 1 < inner_only; ++g) K.cluster_sync[g] = 0;
+            K.sync_stages = B + std::min(inner_only, 1);
         }
         // sweep order: stage-major, CTA of the bisection, definition order
         auto& order = k == 0 ? S.distance_order : (k == 1 ? S.dihedral_order : S.membrane_order);
@@ -1000,7 +994,6 @@ void verify_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_
             int k, s;
             global_stage(S, g, k, s);
             if (stage_touches(d, S, attached, g)) fail("line iteration window touches a suspension node");
-            if (!S.kinds[k].cluster_sync[s]) fail("line iteration window without cluster barriers");
             const size_t o = static_cast<size_t>(S.susp_cta) * (S.kinds[k].stages + 1) + s;
             if (S.kinds[k].offsets[o + 1] - S.kinds[k].offsets[o] > S.line_owner_records)
                 fail("line iteration window record count");
@@ -1008,16 +1001,10 @@ void verify_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_
     }
     std::vector<int64_t> stamp(N, -1);
     int64_t epoch = 0;
-    // runs of stages joined by CTA barriers: a node may be touched by one CTA only
-    std::vector<int64_t> run_of(N, -1);
-    std::vector<int> run_cta(N, -1);
-    int64_t run = 0;
     for (int k = 0; k < 3; ++k) {
         const ClusterKind& K = S.kinds[k];
         const size_t m = k == 0 ? d.constraints.size() : (k == 1 ? d.dihedrals.size() : d.membranes.size());
         std::vector<uint8_t> seen(m, 0);
-        if (K.cluster_sync.size() != static_cast<size_t>(K.stages)) fail("barrier kinds per stage");
-        if (K.stages > 0 && !K.cluster_sync.back()) fail("a kind must end with a cluster barrier");
         for (int s = 0; s < K.stages; ++s) {
             ++epoch;
             for (int c = 0; c < C; ++c)
@@ -1035,13 +1022,8 @@ void verify_cluster_schedule(const OwnedDefinition& d, const std::vector<uint32_
                         if (n != want[q]) fail("reference does not name the constraint's node");
                         if (stamp[n] == epoch) fail("stage is not node-disjoint");
                         stamp[n] = epoch;
-                        if (run_of[n] == run && run_cta[n] != c)
-                            fail("a node is touched by two CTAs between cluster barriers");
-                        run_of[n] = run;
-                        run_cta[n] = c;
                     }
                 }
-            if (K.cluster_sync[s]) ++run;
         }
         for (size_t i = 0; i < m; ++i)
             if (!seen[i]) fail("constraint not scheduled");

@@ -73,10 +73,8 @@ struct ClusterKind {
     std::vector<float> comp;     // distance: sign bit = cable
     std::vector<uint32_t> def_index;
     uint32_t max_cta_records = 0;  // multipliers held in shared memory per CTA
-    std::vector<uint8_t> cluster_sync;  // [stages]: 1 = cluster barrier after the stage, 0 = CTA barrier
-    // split stages: the first interior_stages stages hold only records whose
-    // nodes all lie in the executing CTA's patch; boundary_stages follow
-    int interior_stages = 0, boundary_stages = 0;
+    int sync_stages = 0;  // stages after which nodes may change hands (split stages: those with
+                          // records that span CTAs, and the last one before them)
 };
 
 // Where a record sends a node after its projection: 0 = nowhere (the node
@@ -169,12 +167,11 @@ inline void global_stage(const ClusterSchedule& s, int g, int& kind, int& local)
     }
 }
 
-// Stages of an iteration whose records may span CTAs (after which nodes
-// change hands), plus the line iteration where it follows the stages.
+// Stages of an iteration after which nodes may change hands, plus the line
+// iteration where it follows the stages.
 inline int cluster_barriers_per_iteration(const ClusterSchedule& s) {
     int n = s.susp_cta >= 0 && s.line_stage < 0 ? 1 : 0;
-    for (const ClusterKind& k : s.kinds)
-        for (uint8_t b : k.cluster_sync) n += b;
+    for (const ClusterKind& k : s.kinds) n += k.sync_stages;
     return n;
 }
 

@@ -654,7 +654,7 @@ void StructureImpl::setup_contact(const swb_solver_options& opt) {
     c.lv_succ = dalloc<uint32_t>(owned, 6 * cap);
     c.lv_nsucc = dalloc<uint32_t>(owned, cap);
     c.lv_npred = dalloc<uint32_t>(owned, cap);
-    c.lv_front = dalloc<uint32_t>(owned, 2 * cap);
+    c.lv_front = dalloc<uint32_t>(owned, cap);
     c.fail = dalloc<unsigned long long>(owned, 1);
     cuda_check(cudaMemsetAsync(c.fail, 0xff, sizeof(unsigned long long), stream), "memset");
     d_contact = dupload(owned, std::vector<ContactDev>{c}, stream);
